@@ -5,7 +5,9 @@
 Compiles every csrc/*.cu with nvcc (one process per file, in parallel) and links
 lib/libqfactory_b200.so.  The library only depends on the statically linked CUDA
 runtime, so it loads on a machine without a GPU (calls then fail with a CUDA error).
-A source newer than the library triggers a rebuild.
+csrc/qfb_torch.cpp, the CPython module that calls the library on torch tensors, is
+compiled with g++ against the installed torch's headers into lib/_qfb_torch.so.
+A source newer than its library triggers a rebuild.
 """
 from __future__ import annotations
 
@@ -13,6 +15,7 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -20,6 +23,9 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libqfactory_b200.so")
+TORCH_SRC = os.path.join(CSRC, "qfb_torch.cpp")
+TORCH_LIB = os.path.join(LIB_DIR, "_qfb_torch.so")
+HEADER = os.path.join(os.path.dirname(HERE), "include", "qfactory_b200.h")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -41,8 +47,7 @@ def sources() -> list[str]:
 
 
 def _deps() -> list[str]:
-    inc = os.path.join(os.path.dirname(HERE), "include", "qfactory_b200.h")
-    return sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + [inc]
+    return sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + [HEADER]
 
 
 def is_stale() -> bool:
@@ -52,7 +57,31 @@ def is_stale() -> bool:
     return any(os.path.getmtime(d) > t for d in _deps())
 
 
+def build_torch_module(force: bool = False, verbose: bool = False) -> str:
+    if not force and os.path.exists(TORCH_LIB) and all(
+            os.path.getmtime(d) <= os.path.getmtime(TORCH_LIB) for d in (TORCH_SRC, HEADER)):
+        return TORCH_LIB
+    import torch
+
+    os.makedirs(LIB_DIR, exist_ok=True)
+    root = os.path.dirname(torch.__file__)
+    cuda_inc = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
+    tmp = TORCH_LIB + ".tmp"
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I" + os.path.join(root, "include"), "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           "-I" + sysconfig.get_paths()["include"], "-I" + (cuda_inc if os.path.isdir(cuda_inc) else "/usr/local/cuda/include"),
+           TORCH_SRC, "-o", tmp, "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on {TORCH_SRC}")
+    os.replace(tmp, TORCH_LIB)
+    return TORCH_LIB
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
+    build_torch_module(force, verbose)
     if not force and not is_stale():
         return LIB
     os.makedirs(OBJ, exist_ok=True)

@@ -12,6 +12,7 @@ import os
 
 _PKG_ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 LIB_PATH = os.path.join(_PKG_ROOT, "lib", "libqfactory_b200.so")
+TORCH_MODULE_PATH = os.path.join(_PKG_ROOT, "lib", "_qfb_torch.so")
 
 QFB_OK = 0
 FLAG_PDL = 1
@@ -185,6 +186,49 @@ def lib() -> ctypes.CDLL:
     L.qfb_comm_last_cuda_error.restype = i32
     _lib = L
     return L
+
+
+_torch_module = None
+_layer_types = ()
+
+
+def serve_types(*types) -> None:
+    """Layer classes whose `__call__` becomes the native one when the module below is loaded (exactly these
+    classes: a subclass may bring a `forward` of its own)."""
+    global _layer_types
+    _layer_types = types
+
+
+def torch_module():
+    """The CPython module that runs the hot calls on torch tensors (csrc/qfb_torch.cpp), loaded and bound to the
+    library once; raises when it has not been built."""
+    global _torch_module
+    if _torch_module is None:
+        import importlib.machinery
+        import importlib.util
+
+        import torch.nn.modules.module as tm
+
+        if not os.path.exists(TORCH_MODULE_PATH):
+            raise NativeError(f"native module {TORCH_MODULE_PATH} not found: build it with "
+                              f"`python {os.path.join(_PKG_ROOT, 'build.py')}`; there is no fallback path")
+        loader = importlib.machinery.ExtensionFileLoader("_qfb_torch", TORCH_MODULE_PATH)
+        spec = importlib.util.spec_from_file_location("_qfb_torch", TORCH_MODULE_PATH, loader=loader)
+        m = importlib.util.module_from_spec(spec)
+        loader.exec_module(m)
+        L = lib()
+        names = ("qfb_linear_forward", "qfb_linear_silu_mul_forward", "qfb_rmsnorm", "qfb_add_rmsnorm", "qfb_silu_mul",
+                 "qfb_decode_attention_rope")
+        # what nn.Module.__call__ looks at before it goes straight to forward: the dictionaries of hooks, torch's own
+        # and the module's
+        hooks = tuple(getattr(tm, n) for n in ("_global_backward_pre_hooks", "_global_backward_hooks", "_global_forward_hooks",
+                                               "_global_forward_pre_hooks"))
+        keys = ("_backward_hooks", "_backward_pre_hooks", "_forward_hooks", "_forward_pre_hooks", "_compiled_call_impl")
+        m.bind({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in names}, tm.Module.__call__, _layer_types, hooks, keys)
+        for t in _layer_types:
+            t.__call__ = m.layer_call_method
+        _torch_module = m
+    return _torch_module
 
 
 def check(status: int, what: str = "qfactory_b200") -> None:

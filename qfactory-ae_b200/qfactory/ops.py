@@ -17,6 +17,9 @@ def _stream(t):
 
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5, out: torch.Tensor | None = None) -> torch.Tensor:
     """fp16(x * rsqrt(mean(x^2, -1) + eps)) * weight over the last dimension."""
+    y = _native.torch_module().rmsnorm(x, None, weight, eps, out)
+    if isinstance(y, torch.Tensor):
+        return y
     assert x.is_cuda and x.dtype == torch.float16 and x.is_contiguous() and weight.dtype == torch.float16
     d = x.shape[-1]
     if out is None:
@@ -29,6 +32,9 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5, out: torch
 def add_rmsnorm(x: torch.Tensor, residual: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5,
                 out: torch.Tensor | None = None) -> torch.Tensor:
     """x += residual (in place, fp16), then the RMS norm of the sum: returns the normed tensor."""
+    y = _native.torch_module().rmsnorm(x, residual, weight, eps, out)
+    if isinstance(y, torch.Tensor):
+        return y
     assert x.is_cuda and x.dtype == torch.float16 and x.is_contiguous()
     assert residual.shape == x.shape and residual.dtype == torch.float16 and residual.is_contiguous()
     d = x.shape[-1]
@@ -41,6 +47,9 @@ def add_rmsnorm(x: torch.Tensor, residual: torch.Tensor, weight: torch.Tensor, e
 
 def silu_mul(gate_up: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
     """silu(gate_up[..., :h]) * gate_up[..., h:] with h = half of the last dimension."""
+    y = _native.torch_module().silu_mul(gate_up, out)
+    if isinstance(y, torch.Tensor):
+        return y
     assert gate_up.is_cuda and gate_up.dtype == torch.float16 and gate_up.is_contiguous()
     half = gate_up.shape[-1] // 2
     rows = gate_up.numel() // (2 * half)
@@ -94,6 +103,9 @@ def decode_attention_rope(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tenso
     """`rope_cache` and `decode_attention` of ONE new token per batch row in one launch: qkv
     [B, 1, q_heads + 2 kv_heads, hd] un-rotated (and left so); the rotated key and the value are written
     into the caches at pos [1]; returns [B, q_heads * hd].  Bit-identical to the two separate calls."""
+    y = _native.torch_module().decode_attention_rope(qkv, cos, sin, pos, k_cache, v_cache, q_heads, kv_heads, out)
+    if isinstance(y, torch.Tensor):
+        return y
     B, T, H, hd = qkv.shape
     assert T == 1 and H == q_heads + 2 * kv_heads and qkv.is_contiguous() and qkv.dtype == torch.float16
     assert pos.dtype == torch.int64 and pos.numel() == 1 and k_cache.is_contiguous() and v_cache.is_contiguous()

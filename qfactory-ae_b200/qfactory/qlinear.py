@@ -39,7 +39,8 @@ class _PackedLinear(torch.nn.Module):
         self.register_buffer("w", w)
         self.register_buffer("s", s)
         self.register_buffer("z", z)
-        self.flags = 0
+        self._native_call = None   # the C++ call object (_native.torch_module), made by _prepare
+        self._flags = 0
         self._desc = None
         self._ws = None
         self._ws_bytes = 0
@@ -56,6 +57,29 @@ class _PackedLinear(torch.nn.Module):
         # the workspace pointer handed to the hot call follows the tensor
         self._ws_tensor = t
         self._ws_ptr = t.data_ptr() if t is not None else None
+        if self._native_call is not None:
+            self._native_call.ws_ptr = self._ws_ptr or 0
+
+    @property
+    def _ws_bytes(self):
+        return self._ws_size
+
+    @_ws_bytes.setter
+    def _ws_bytes(self, n):
+        self._ws_size = n
+        if self._native_call is not None:
+            self._native_call.ws_bytes = n
+
+    @property
+    def flags(self):
+        """QFB_FLAG_* of every call of this layer."""
+        return self._flags
+
+    @flags.setter
+    def flags(self, f):
+        self._flags = f
+        if self._native_call is not None:
+            self._native_call.flags = f
 
     def _prepare(self):
         if not self.w.is_cuda:
@@ -75,6 +99,10 @@ class _PackedLinear(torch.nn.Module):
         # pre-resolved pieces of the hot call
         self._desc_ref = ctypes.byref(d)
         self._fwd = L.qfb_linear_forward
+        silu_rows = (8 if self.n_bits == 3 else 16) if self.packed_layout == layout.LAYOUT_FRAGMENT else 0
+        self._native_call = _native.torch_module().LayerCall(
+            d.qweight or 0, d.scales or 0, d.zeros or 0, d.n, d.k, d.bits, d.group_size, d.layout, self._ws_ptr, nbytes,
+            self._flags, silu_rows, self.w.get_device(), (self.w, self.s, self.z))
 
     # -- the packed layout travels with the checkpoint ------------------------
     def get_extra_state(self):
@@ -94,12 +122,17 @@ class _PackedLinear(torch.nn.Module):
     def _apply(self, fn, *a, **kw):
         r = super()._apply(fn, *a, **kw)
         self._desc = None  # device pointers changed
+        self._native_call = None
         self._host = None
         return r
 
     def forward(self, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         if self._desc is None:
             self._prepare()
+        y = self._native_call.forward(x, out)
+        if isinstance(y, torch.Tensor):
+            return y
+        # the general path: other ranks and strides, other devices, and the errors
         K, N = self.in_features, self.out_features
         assert x.dtype == torch.float16, "activations must be fp16"
         assert x.shape[-1] == K
@@ -166,6 +199,9 @@ class _PackedLinear(torch.nn.Module):
         element-wise kernel followed by `forward`.  Both give the same bits."""
         if self._desc is None:
             self._prepare()
+        y = self._native_call.forward_silu_mul(gate_up, out)
+        if isinstance(y, torch.Tensor):
+            return y
         assert gate_up.dtype == torch.float16 and gate_up.shape[-1] == 2 * self.in_features
         g2 = gate_up.reshape(-1, 2 * self.in_features)
         if not g2.is_contiguous():
@@ -289,6 +325,9 @@ class GEMVLinear(_PackedLinear):
         assert w.numel() == layout.padded_rows(out_features) * in_features * n_bits // 8
         super().__init__(in_features, out_features, n_bits, -1, w, None, None, max_batch=max(16, batch_size),
                          packed_layout=lay)
+
+
+_native.serve_types(GPTQLinear, GEMVLinear)
 
 
 class QLinear:
