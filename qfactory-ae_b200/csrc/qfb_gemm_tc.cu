@@ -61,7 +61,12 @@ struct TcCfg {
   static constexpr int kXStages = (kTwoPerSM && !POST) ? (NB <= 32 ? 6 : NB <= 64 ? 3 : 2)
                                   : NB <= 16 ? 6 : NB <= 32 ? (POST ? 4 : 8) : NB <= 64 ? 6 : NB <= 128 ? 4 : (BITS == 8 ? 2 : 3);
   static constexpr int kWStagesRaw = (kBudget - kXStages * kXBytes) / (kWBytes + kQBytes);
-  static constexpr int kWStages = kWStagesRaw > 16 ? 16 : kWStagesRaw;
+  // with two decode groups an even number of slots: a wait on the parity of a full barrier is only sound for a thread
+  // that knows the phase before the awaited one to be complete, and with an odd number the previous stage in a slot
+  // belongs to the other group, whose bulk copy may land later than the copies after it (the wait then fell through
+  // and the group decoded a slot that was still being filled)
+  static constexpr int kWStagesCap = kWStagesRaw > 16 ? 16 : kWStagesRaw;
+  static constexpr int kWStages = DG == 2 ? kWStagesCap & ~1 : kWStagesCap;
   static constexpr int kTmemCols = kTwoPerSM ? 256 : 512;
   // ring of R slots in tensor memory: A operand (64 columns) + in POST mode one accumulator each
   static constexpr int kSlotCols = kAColsPerSlot + (POST ? NB : 0);
@@ -461,8 +466,10 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const TcParams p) {
       for (int i = e; i < nkb; i += Cfg::kIssuers) {
         const int xs = i % NX, r = i % R;
         const uint32_t phx = (uint32_t)(i / NX) & 1u, phr = (uint32_t)(i / R) & 1u;
-        if (!mbar_wait(smem_u32(&bar_xfull[xs]), phx, abortp, kSleepMma, wait_limit)) break;
+        // (the operand in tensor memory first: its decode waited for the MMAs of stage i - R, so the previous stage in
+        // the activation slot, which may be the other issuer's, has landed and the parity of xfull is unambiguous)
         if (!mbar_wait(smem_u32(&bar_afull[r]), phr, abortp, kSleepMma, wait_limit)) break;
+        if (!mbar_wait(smem_u32(&bar_xfull[xs]), phx, abortp, kSleepMma, wait_limit)) break;
         if (POST) {
           if (!mbar_wait(smem_u32(&bar_dempty[r]), phr ^ 1u, abortp, kSleepMma, wait_limit)) break;
         }
