@@ -65,8 +65,10 @@ typedef enum qfb_status {
 } qfb_status;
 
 /* flags for qfb_linear_forward */
-#define QFB_FLAG_PDL 1u          /* launch with programmatic stream serialisation: the kernel
-                                    prefetches weights before it waits for the preceding kernel */
+#define QFB_FLAG_PDL 1u          /* the kernel prefetches weights before it waits for the preceding
+                                    kernel: nothing still running in the stream writes them.  (Every
+                                    launch uses programmatic stream serialisation; without the flag
+                                    the wait comes before the first read.) */
 #define QFB_FLAG_FORCE_SIMT 2u   /* never the tcgen05 kernel: tile-layout layers run the CUDA-core
                                     split-K kernel, fragment-layout layers the mma.sync GEMV (in
                                     passes of 16 rows), whatever the batch size */

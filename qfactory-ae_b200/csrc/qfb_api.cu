@@ -248,6 +248,7 @@ static int run_tc(const LayerView& v, const __half* x, int m, __half* y, void* w
   p.steps_per_group = gs / 16;
   p.halfstages_per_group = gs / 64;
   p.zconst = v.zconst;
+  p.early = (flags & QFB_FLAG_PDL) ? 1 : 0;
   p.layout = v.layout;
   p.partial = nullptr;
   p.counters = nullptr;
@@ -284,7 +285,7 @@ static int run_tc(const LayerView& v, const __half* x, int m, __half* y, void* w
   tl_last_launch[2] = p.tail_split > 1 ? p.tail_split : grid.z;
   tl_last_launch[3] = 256 + 256 * pl.dg;
   tl_last_launch[4] = pl.nb;
-  return check_cuda(launch_gemm_tc(tm, p, v.bits, pl.nb, pl.post, pl.dg, grid, (flags & QFB_FLAG_PDL) != 0, st));
+  return check_cuda(launch_gemm_tc(tm, p, v.bits, pl.nb, pl.post, pl.dg, grid, st));
 }
 
 static int choose_kernel(const LayerView& v, int m, unsigned flags) {
@@ -345,6 +346,7 @@ static int run_gemv(const LayerView& v, const __half* x, int m, __half* y, void*
     p.max_units_per_cta = (v.units + pl.split - 1) / pl.split;
     p.units_per_kway = (p.max_units_per_cta + pl.kways - 1) / pl.kways;
     p.zconst = v.zconst;
+  p.early = (flags & QFB_FLAG_PDL) ? 1 : 0;
     p.partial = nullptr;
     p.counters = nullptr;
     if (pl.split > 1) {
@@ -361,7 +363,7 @@ static int run_gemv(const LayerView& v, const __half* x, int m, __half* y, void*
     tl_last_launch[2] = grid.y;
     tl_last_launch[3] = block;
     tl_last_launch[4] = (int)pl.smem;
-    int stt = check_cuda(launch_gemv(p, v.bits, pl.mb, grid, block, pl.smem, (flags & QFB_FLAG_PDL) != 0, st));
+    int stt = check_cuda(launch_gemv(p, v.bits, pl.mb, grid, block, pl.smem, st));
     if (stt != QFB_OK) return stt;
   }
   return QFB_OK;
@@ -531,6 +533,7 @@ static int run_mma(const LayerView& v, const __half* x, int m, __half* y, void* 
     p.batches_div = p.batches / pl.split;
     p.batches_mod = p.batches % pl.split;
     p.zconst = v.zconst;
+    p.early = (flags & QFB_FLAG_PDL) ? 1 : 0;
     p.partial = nullptr;
     p.counters = nullptr;
     // up to 8 splits reduce inside a thread-block cluster; more go through the workspace
@@ -553,7 +556,7 @@ static int run_mma(const LayerView& v, const __half* x, int m, __half* y, void* 
     tl_last_launch[2] = grid.y;
     tl_last_launch[3] = block;
     tl_last_launch[4] = (int)pl.smem;
-    cudaError_t ce = launch_gemv_mma(p, v.bits, pl.nt, grid, block, pl.smem, (flags & QFB_FLAG_PDL) != 0, st);
+    cudaError_t ce = launch_gemv_mma(p, v.bits, pl.nt, grid, block, pl.smem, st);
     if (ce != cudaSuccess && p.cluster) {
       // a cluster launch the device refuses (e.g. a partitioned GPU): same split through the workspace
       (void)cudaGetLastError();
@@ -563,7 +566,7 @@ static int run_mma(const LayerView& v, const __half* x, int m, __half* y, void* 
         p.cluster = 0;
         p.counters = reinterpret_cast<unsigned*>(static_cast<char*>(workspace) + kHeaderBytes);
         p.partial = reinterpret_cast<float*>(static_cast<char*>(workspace) + off);
-        ce = launch_gemv_mma(p, v.bits, pl.nt, grid, block, pl.smem, (flags & QFB_FLAG_PDL) != 0, st);
+        ce = launch_gemv_mma(p, v.bits, pl.nt, grid, block, pl.smem, st);
       }
     }
     const int stt = check_cuda(ce);

@@ -399,13 +399,14 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const TcParams p) {
   volatile int* abortp = &abort_flag;
   const long long wait_limit = p.stall_test ? 200000LL : kWaitLimitCycles;
   grid_launch_dependents();
+  if (!p.early) grid_dependency_wait();
 
   const bool has_z = ASYM || p.qz != nullptr;
   const bool has_s = ASYM || p.qs != nullptr;
 
   if (warp == 0) {
     // ------------------------------ weight producer ---------------------------
-    // (never depends on the preceding kernel: no dependency wait on this path)
+    // (depends on the preceding kernel only where TcParams::early is not set: the wait above)
     if (lane == 0) {
       const uint8_t* wsrc = reinterpret_cast<const uint8_t*>(p.qw) + ((size_t)tile * p.kblocks + kb0) * Cfg::kWBytes;
       int s = 0;
@@ -667,16 +668,16 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const TcParams p) {
 // host side
 // ---------------------------------------------------------------------------------------
 template <int BITS, int NB, bool POST, int DG, bool FRAG>
-static cudaError_t launch_cfg_layout(const CUtensorMap& tm, const TcParams& p, dim3 grid, bool pdl, cudaStream_t st);
+static cudaError_t launch_cfg_layout(const CUtensorMap& tm, const TcParams& p, dim3 grid, cudaStream_t st);
 
 template <int BITS, int NB, bool POST, int DG>
-static cudaError_t launch_cfg(const CUtensorMap& tm, const TcParams& p, dim3 grid, bool pdl, cudaStream_t st) {
-  if (p.layout == QFB_LAYOUT_FRAGMENT) return launch_cfg_layout<BITS, NB, POST, DG, true>(tm, p, grid, pdl, st);
-  return launch_cfg_layout<BITS, NB, POST, DG, false>(tm, p, grid, pdl, st);
+static cudaError_t launch_cfg(const CUtensorMap& tm, const TcParams& p, dim3 grid, cudaStream_t st) {
+  if (p.layout == QFB_LAYOUT_FRAGMENT) return launch_cfg_layout<BITS, NB, POST, DG, true>(tm, p, grid, st);
+  return launch_cfg_layout<BITS, NB, POST, DG, false>(tm, p, grid, st);
 }
 
 template <int BITS, int NB, bool POST, int DG, bool FRAG>
-static cudaError_t launch_cfg_layout(const CUtensorMap& tm, const TcParams& p, dim3 grid, bool pdl, cudaStream_t st) {
+static cudaError_t launch_cfg_layout(const CUtensorMap& tm, const TcParams& p, dim3 grid, cudaStream_t st) {
   using Cfg = TcCfg<BITS, NB, POST, DG>;
   auto kern = qgemm_tc_kernel<BITS, NB, POST, DG, FRAG, false>;
   // scale-in-the-decode mode: the common case of scales and zero points present has a build of its own (measured:
@@ -696,48 +697,48 @@ static cudaError_t launch_cfg_layout(const CUtensorMap& tm, const TcParams& p, d
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, tm, p);
 }
 
 template <int BITS, int DG>
-static cudaError_t launch_nb(const CUtensorMap& tm, const TcParams& p, int nb, bool post, dim3 grid, bool pdl,
+static cudaError_t launch_nb(const CUtensorMap& tm, const TcParams& p, int nb, bool post, dim3 grid,
                              cudaStream_t st) {
   if (post) {
     if (DG != 1) return cudaErrorInvalidValue;  // (narrow batch tiles: one decode group only)
     switch (nb) {
-      case 16: return launch_cfg<BITS, 16, true, 1>(tm, p, grid, pdl, st);
-      case 32: return launch_cfg<BITS, 32, true, 1>(tm, p, grid, pdl, st);
+      case 16: return launch_cfg<BITS, 16, true, 1>(tm, p, grid, st);
+      case 32: return launch_cfg<BITS, 32, true, 1>(tm, p, grid, st);
       default: return cudaErrorInvalidValue;
     }
   }
   switch (nb) {
-    case 64: return launch_cfg<BITS, 64, false, DG>(tm, p, grid, pdl, st);
-    case 128: return launch_cfg<BITS, 128, false, DG>(tm, p, grid, pdl, st);
-    case 256: return launch_cfg<BITS, 256, false, DG>(tm, p, grid, pdl, st);
+    case 64: return launch_cfg<BITS, 64, false, DG>(tm, p, grid, st);
+    case 128: return launch_cfg<BITS, 128, false, DG>(tm, p, grid, st);
+    case 256: return launch_cfg<BITS, 256, false, DG>(tm, p, grid, st);
     default: return cudaErrorInvalidValue;
   }
 }
 
 template <int DG>
 static cudaError_t launch_bits(const CUtensorMap& tmap_x, const TcParams& p, int bits, int nb, bool post, dim3 grid,
-                               bool pdl, cudaStream_t st) {
+                               cudaStream_t st) {
   switch (bits) {
-    case 2: return launch_nb<2, DG>(tmap_x, p, nb, post, grid, pdl, st);
-    case 3: return launch_nb<3, DG>(tmap_x, p, nb, post, grid, pdl, st);
-    case 4: return launch_nb<4, DG>(tmap_x, p, nb, post, grid, pdl, st);
-    case 8: return launch_nb<8, DG>(tmap_x, p, nb, post, grid, pdl, st);
+    case 2: return launch_nb<2, DG>(tmap_x, p, nb, post, grid, st);
+    case 3: return launch_nb<3, DG>(tmap_x, p, nb, post, grid, st);
+    case 4: return launch_nb<4, DG>(tmap_x, p, nb, post, grid, st);
+    case 8: return launch_nb<8, DG>(tmap_x, p, nb, post, grid, st);
     default: return cudaErrorInvalidValue;
   }
 }
 
 cudaError_t launch_gemm_tc(const CUtensorMap& tmap_x, const TcParams& p, int bits, int nb, bool post, int decode_groups,
-                           dim3 grid, bool pdl, cudaStream_t st) {
+                           dim3 grid, cudaStream_t st) {
   // two decode groups (768 threads, one CTA per SM) where the scale is applied in the decode:
   // measured +10-17 % from 33 rows up, bit-identical results; three groups (1024 threads, 64
   // registers) were 3-6 % slower than two, and the narrow per-stage-accumulator tiles gain nothing
-  if (decode_groups == 2 && !post) return launch_bits<2>(tmap_x, p, bits, nb, post, grid, pdl, st);
-  return launch_bits<1>(tmap_x, p, bits, nb, post, grid, pdl, st);
+  if (decode_groups == 2 && !post) return launch_bits<2>(tmap_x, p, bits, nb, post, grid, st);
+  return launch_bits<1>(tmap_x, p, bits, nb, post, grid, st);
 }
 
 }  // namespace qfb

@@ -84,6 +84,7 @@ __global__ void __launch_bounds__(256, (MB <= 2 ? 3 : 2)) gemv_splitk_kernel(con
     }
   };
 
+  if (!p.early) grid_dependency_wait();
   load_batch(tb);
   grid_launch_dependents();
   grid_dependency_wait();
@@ -221,7 +222,7 @@ __global__ void __launch_bounds__(256, (MB <= 2 ? 3 : 2)) gemv_splitk_kernel(con
 }
 
 template <int BITS, int MB>
-static cudaError_t launch_one(const GemvParams& p, dim3 grid, int block, size_t smem, bool pdl, cudaStream_t st) {
+static cudaError_t launch_one(const GemvParams& p, dim3 grid, int block, size_t smem, cudaStream_t st) {
   constexpr int U = (BITS == 3) ? 2 : (BITS == 2 ? 4 : 8);
   auto kern = gemv_splitk_kernel<BITS, MB, U>;
   cudaLaunchConfig_t cfg = {};
@@ -233,7 +234,7 @@ static cudaError_t launch_one(const GemvParams& p, dim3 grid, int block, size_t 
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cfg.numAttrs = 1;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -242,23 +243,23 @@ static cudaError_t launch_one(const GemvParams& p, dim3 grid, int block, size_t 
 }
 
 template <int BITS>
-static cudaError_t launch_bits(const GemvParams& p, int mb, dim3 grid, int block, size_t smem, bool pdl,
+static cudaError_t launch_bits(const GemvParams& p, int mb, dim3 grid, int block, size_t smem,
                                cudaStream_t st) {
   switch (mb) {
-    case 1: return launch_one<BITS, 1>(p, grid, block, smem, pdl, st);
-    case 2: return launch_one<BITS, 2>(p, grid, block, smem, pdl, st);
-    case 4: return launch_one<BITS, 4>(p, grid, block, smem, pdl, st);
-    default: return launch_one<BITS, 8>(p, grid, block, smem, pdl, st);
+    case 1: return launch_one<BITS, 1>(p, grid, block, smem, st);
+    case 2: return launch_one<BITS, 2>(p, grid, block, smem, st);
+    case 4: return launch_one<BITS, 4>(p, grid, block, smem, st);
+    default: return launch_one<BITS, 8>(p, grid, block, smem, st);
   }
 }
 
-cudaError_t launch_gemv(const GemvParams& p, int bits, int mb, dim3 grid, int block, size_t smem, bool pdl,
+cudaError_t launch_gemv(const GemvParams& p, int bits, int mb, dim3 grid, int block, size_t smem,
                         cudaStream_t st) {
   switch (bits) {
-    case 2: return launch_bits<2>(p, mb, grid, block, smem, pdl, st);
-    case 3: return launch_bits<3>(p, mb, grid, block, smem, pdl, st);
-    case 4: return launch_bits<4>(p, mb, grid, block, smem, pdl, st);
-    case 8: return launch_bits<8>(p, mb, grid, block, smem, pdl, st);
+    case 2: return launch_bits<2>(p, mb, grid, block, smem, st);
+    case 3: return launch_bits<3>(p, mb, grid, block, smem, st);
+    case 4: return launch_bits<4>(p, mb, grid, block, smem, st);
+    case 8: return launch_bits<8>(p, mb, grid, block, smem, st);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -29,8 +29,8 @@
 // workspace by the last CTA of the tile to arrive; both in split order (deterministic; the
 // counters reset themselves).
 //
-// Ordering under programmatic dependent launch: weight, scale and zero loads are issued before
-// griddepcontrol.wait; activations, workspace and output are only touched after it.
+// Ordering under programmatic dependent launch: with MmaParams::early weight, scale and zero loads are issued
+// before griddepcontrol.wait, otherwise after it; activations, workspace and output are only touched after it.
 #include <map>
 #include <mutex>
 
@@ -232,6 +232,7 @@ __device__ __forceinline__ void gemv_mma_body(const MmaParams& p) {
   for (int i = 0; i < RB / 2; ++i) sz_cur.z[i] = 0;
   auto sz_offset = [&](int gi) { return (((size_t)tile * p.groups + gi) * 2 + wt) * 64 + g * 8 + sub * 4; };
 
+  if (!p.early) grid_dependency_wait();
   Words<NW> w[NSLOT][8];
 #pragma unroll
   for (int sl = 0; sl < NSLOT; ++sl)
@@ -784,7 +785,7 @@ __global__ void __launch_bounds__(128, 5) gemv_mma_kernel_small(const MmaParams 
 }
 
 template <int BITS, int NT, int RB, bool SEG64>
-static cudaError_t launch_cfg(const MmaParams& p, dim3 grid, int block, size_t smem, bool pdl, cudaStream_t st) {
+static cudaError_t launch_cfg(const MmaParams& p, dim3 grid, int block, size_t smem, cudaStream_t st) {
   auto kern = block <= kMmaSmallBlock ? gemv_mma_kernel_small<BITS, NT, RB, SEG64> : gemv_mma_kernel<BITS, NT, RB, SEG64>;
   if (!p.act && (p.cluster || grid.x == 1) && !p.push.world) {
     kern = block <= kMmaSmallBlock ? gemv_mma_kernel_small<BITS, NT, RB, SEG64, false, true>
@@ -839,12 +840,9 @@ static cudaError_t launch_cfg(const MmaParams& p, dim3 grid, int block, size_t s
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
-  int na = 0;
-  if (pdl) {
-    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[na].val.programmaticStreamSerializationAllowed = 1;
-    ++na;
-  }
+  int na = 1;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
   if (p.cluster) {  // the K splits of one tile form a cluster
     attr[na].id = cudaLaunchAttributeClusterDimension;
     attr[na].val.clusterDim.x = grid.x;
@@ -928,10 +926,10 @@ int mma_max_active_clusters(int bits, int nt, bool seg64, int block, size_t smem
   return n;
 }
 
-cudaError_t launch_gemv_mma(const MmaParams& p, int bits, int nt, dim3 grid, int block, size_t smem, bool pdl,
+cudaError_t launch_gemv_mma(const MmaParams& p, int bits, int nt, dim3 grid, int block, size_t smem,
                             cudaStream_t st) {
   const bool seg64 = p.chunks_per_group == 1;
-  QFB_MMA_DISPATCH(launch_cfg, p, grid, block, smem, pdl, st);
+  QFB_MMA_DISPATCH(launch_cfg, p, grid, block, smem, st);
   return cudaErrorInvalidValue;
 }
 
