@@ -222,6 +222,21 @@ int qfb_pack(const int32_t* codes, const void* scales, const int32_t* zeros, int
 int qfb_pack_layout(const int32_t* codes, const void* scales, const int32_t* zeros, int n, int k,
                     int bits, int group_size, int layout, void* qweight_out, void* scales_out,
                     void* zeros_out, void* stream);
+/* qfb_pack_layout that also reports values outside 0 .. 2^bits - 1: bit 0 (a code) and bit 1 (a zero
+ * point) are set in the device word *range_flags (zeroed by the caller; may be NULL). */
+int qfb_pack_checked(const int32_t* codes, const void* scales, const int32_t* zeros, int n, int k,
+                     int bits, int group_size, int layout, void* qweight_out, void* scales_out,
+                     void* zeros_out, unsigned* range_flags, void* stream);
+/* Packs a GPTQ checkpoint's own tensors (2, 4, 8 bits): qweight i32 [k / (32/bits), n], scales f16
+ * [k/group, n], qzeros i32 [k/group, zero_words] (NULL: symmetric), fields as in the checkpoint, without
+ * an unpacked copy in between. */
+int qfb_pack_gptq(const void* qweight, const void* scales, const void* qzeros, int zero_words, int n,
+                  int k, int bits, int group_size, int layout, void* qweight_out, void* scales_out,
+                  void* zeros_out, void* stream);
+/* qfb_quantize followed by qfb_pack_checked, in one pass over the weight (f16 [k, n]). */
+int qfb_quantize_pack(const void* weight, int n, int k, int bits, int group_size, int layout,
+                      void* qweight_out, void* scales_out, void* zeros_out, unsigned* range_flags,
+                      void* stream);
 int qfb_layout_supported(int layout, int n, int k, int bits, int group_size);
 
 /*

@@ -883,35 +883,79 @@ int qfb_pack(const int32_t* codes, const void* scales, const int32_t* zeros, int
                          zeros_out, stream);
 }
 
-int qfb_pack_layout(const int32_t* codes, const void* scales, const int32_t* zeros, int n, int k, int bits,
-                    int group_size, int layout, void* qweight_out, void* scales_out, void* zeros_out,
-                    void* stream) {
+// the checks and the destination that the packing entry points share
+static int pack_params(int n, int k, int bits, int group_size, int layout, void* qweight_out, void* scales_out,
+                       void* zeros_out, unsigned* range_flags, PackParams* p) {
   int st = validate_shape(n, k, bits, group_size);
   if (st != QFB_OK) return st;
   st = validate_layout(layout, k, bits, group_size);
   if (st != QFB_OK) return st;
-  if (!codes || !qweight_out) return QFB_ERR_NULL_POINTER;
-  if (group_size != -1 && (!scales || !scales_out)) return QFB_ERR_NULL_POINTER;
-  if (group_size == -1 && (scales || zeros)) return QFB_ERR_BAD_SHAPE;
-  if (zeros && !zeros_out) return QFB_ERR_NULL_POINTER;
+  if (!qweight_out || (group_size != -1 && !scales_out)) return QFB_ERR_NULL_POINTER;
   if (!aligned16(qweight_out) || !aligned16(scales_out) || !aligned16(zeros_out)) return QFB_ERR_MISALIGNED;
+  *p = PackParams{};
+  p->qw = static_cast<uint32_t*>(qweight_out);
+  p->qs = group_size == -1 ? nullptr : static_cast<__half*>(scales_out);
+  p->range_flags = range_flags;
+  p->n = n;
+  p->k = k;
+  p->bits = bits;
+  p->group_size = group_size == -1 ? k : group_size;
+  p->npad = padded_rows(n);
+  p->tiles = p->npad / kTileRows;
+  p->units = k / unit_k(bits);
+  p->groups = group_size == -1 ? 1 : k / group_size;
+  p->layout = layout;
+  return QFB_OK;
+}
+
+int qfb_pack_checked(const int32_t* codes, const void* scales, const int32_t* zeros, int n, int k, int bits, int group_size,
+                     int layout, void* qweight_out, void* scales_out, void* zeros_out, unsigned* range_flags, void* stream) {
   PackParams p;
+  const int st = pack_params(n, k, bits, group_size, layout, qweight_out, scales_out, zeros_out, range_flags, &p);
+  if (st != QFB_OK) return st;
+  if (!codes || (group_size != -1 && !scales) || (zeros && !zeros_out)) return QFB_ERR_NULL_POINTER;
+  if (group_size == -1 && (scales || zeros)) return QFB_ERR_BAD_SHAPE;
   p.codes = codes;
   p.scales = static_cast<const __half*>(scales);
   p.zeros = zeros;
-  p.qw = static_cast<uint32_t*>(qweight_out);
-  p.qs = group_size == -1 ? nullptr : static_cast<__half*>(scales_out);
   p.qz = zeros ? static_cast<uint8_t*>(zeros_out) : nullptr;
-  p.n = n;
-  p.k = k;
-  p.bits = bits;
-  p.group_size = group_size;
-  p.npad = padded_rows(n);
-  p.tiles = p.npad / kTileRows;
-  p.units = k / unit_k(bits);
-  p.groups = group_size == -1 ? 1 : k / group_size;
-  p.layout = layout;
   return check_cuda(launch_pack(p, static_cast<cudaStream_t>(stream)));
+}
+
+int qfb_pack_layout(const int32_t* codes, const void* scales, const int32_t* zeros, int n, int k, int bits,
+                    int group_size, int layout, void* qweight_out, void* scales_out, void* zeros_out,
+                    void* stream) {
+  return qfb_pack_checked(codes, scales, zeros, n, k, bits, group_size, layout, qweight_out, scales_out, zeros_out, nullptr,
+                          stream);
+}
+
+int qfb_pack_gptq(const void* qweight, const void* scales, const void* qzeros, int zero_words, int n, int k, int bits,
+                  int group_size, int layout, void* qweight_out, void* scales_out, void* zeros_out, void* stream) {
+  PackParams p;
+  const int st = pack_params(n, k, bits, group_size, layout, qweight_out, scales_out, zeros_out, nullptr, &p);
+  if (st != QFB_OK) return st;
+  if (bits == 3) return QFB_ERR_UNSUPPORTED;
+  if (!qweight || !scales || (qzeros && !zeros_out)) return QFB_ERR_NULL_POINTER;
+  if (group_size == -1 || (qzeros && (long long)zero_words * (32 / bits) < n)) return QFB_ERR_BAD_SHAPE;
+  p.gptq_codes = static_cast<const uint32_t*>(qweight);
+  p.gptq_zeros = static_cast<const uint32_t*>(qzeros);
+  p.zero_words = zero_words;
+  p.scales = static_cast<const __half*>(scales);
+  p.qz = qzeros ? static_cast<uint8_t*>(zeros_out) : nullptr;
+  return check_cuda(launch_pack(p, static_cast<cudaStream_t>(stream)));
+}
+
+int qfb_quantize_pack(const void* weight, int n, int k, int bits, int group_size, int layout, void* qweight_out,
+                      void* scales_out, void* zeros_out, unsigned* range_flags, void* stream) {
+  PackParams p;
+  const int st = pack_params(n, k, bits, group_size, layout, qweight_out, scales_out, zeros_out, range_flags, &p);
+  if (st != QFB_OK) return st;
+  if (group_size == -1) return QFB_ERR_BAD_SHAPE;
+  if (!weight || !zeros_out || !range_flags) return QFB_ERR_NULL_POINTER;
+  if (reinterpret_cast<uintptr_t>(weight) & 3u) return QFB_ERR_MISALIGNED;
+  p.weight = static_cast<const __half*>(weight);
+  p.qz = static_cast<uint8_t*>(zeros_out);
+  return check_cuda(launch_quantize_pack(p, static_cast<cudaStream_t>(stream)));
 }
 
 int qfb_quantize(const void* weight, int k, int n, int bits, int group_size, int32_t* codes_out, void* scales_out,

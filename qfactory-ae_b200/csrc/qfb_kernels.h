@@ -166,17 +166,27 @@ cudaError_t launch_decode_attention(const __half* qkv, __half* k_cache, __half* 
 cudaError_t launch_rope_cache(__half* qkv, const __half* cosv, const __half* sinv, const long long* pos, __half* k_cache,
                               __half* v_cache, int B, int T, int hq, int hkv, int hd, int max_len, cudaStream_t st);
 
+// what PackParams::range_flags collects: a code, or a zero point, outside 0 .. 2^bits - 1
+constexpr unsigned kRangeCodes = 1u, kRangeZeros = 2u;
+// where the codes of a layer come from
+constexpr int kPackCodes = 0, kPackGptq = 1;
 struct PackParams {
   const int32_t* codes;   // [k, n]
   const __half* scales;   // [groups, n] or null
   const int32_t* zeros;   // [groups, n] or null
+  const uint32_t* gptq_codes;   // checkpoint words [k / (32 / bits), n] instead of `codes`
+  const uint32_t* gptq_zeros;   // [groups, zero_words] instead of `zeros`
+  int zero_words;
+  const __half* weight;   // [k, n] fp16 (launch_quantize_pack)
   uint32_t* qw;           // packed words
   __half* qs;
   uint8_t* qz;
+  unsigned* range_flags;  // or null
   int n, k, bits, group_size, npad, tiles, units, groups;
   int layout;             // QFB_LAYOUT_TILE or QFB_LAYOUT_FRAGMENT
 };
 cudaError_t launch_pack(const PackParams& p, cudaStream_t st);
+cudaError_t launch_quantize_pack(const PackParams& p, cudaStream_t st);
 
 cudaError_t launch_quantize(const __half* w, int k, int n, int bits, int group_size, int32_t* codes, __half* scales,
                             int32_t* zeros, cudaStream_t st);

@@ -27,7 +27,7 @@ EXPORTS = (
     "qfb_workspace_bytes", "qfb_workspace_init",
     "qfb_linear_forward", "qfb_linear_forward_host", "qfb_linear_silu_mul_forward", "qfb_select_kernel",
     "qfb_set_gemv_tuning", "qfb_get_last_launch", "qfb_set_tensor_min_batch", "qfb_set_tensor_split", "qfb_set_tensor_decode_groups", "qfb_set_tensor_batch_tile", "qfb_set_cluster_reduce", "qfb_read_status",
-    "qfb_pack", "qfb_pack_layout", "qfb_layout_supported", "qfb_unpack_codes", "qfb_dequantize",
+    "qfb_pack", "qfb_pack_layout", "qfb_pack_checked", "qfb_pack_gptq", "qfb_quantize_pack", "qfb_layout_supported", "qfb_unpack_codes", "qfb_dequantize",
     "qfb_gemv_forward_static", "qfb_static_scratch_capacity",
     "qfb_rmsnorm", "qfb_add_rmsnorm", "qfb_silu_mul", "qfb_rope_cache", "qfb_quantize", "qfb_decode_attention", "qfb_decode_attention_rope",
     "qfb_comm_buffer_bytes", "qfb_comm_max_rows", "qfb_comm_alloc", "qfb_comm_free", "qfb_comm_open", "qfb_comm_close",
@@ -113,6 +113,12 @@ def lib() -> ctypes.CDLL:
     L.qfb_pack.argtypes = [vp, vp, vp, i32, i32, i32, i32, vp, vp, vp, vp]
     L.qfb_pack_layout.restype = i32
     L.qfb_pack_layout.argtypes = [vp, vp, vp, i32, i32, i32, i32, i32, vp, vp, vp, vp]
+    L.qfb_pack_checked.restype = i32
+    L.qfb_pack_checked.argtypes = [vp, vp, vp, i32, i32, i32, i32, i32, vp, vp, vp, vp, vp]
+    L.qfb_pack_gptq.restype = i32
+    L.qfb_pack_gptq.argtypes = [vp, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp]
+    L.qfb_quantize_pack.restype = i32
+    L.qfb_quantize_pack.argtypes = [vp, i32, i32, i32, i32, i32, vp, vp, vp, vp, vp]
     L.qfb_layout_supported.restype = i32
     L.qfb_layout_supported.argtypes = [i32, i32, i32, i32, i32]
     L.qfb_unpack_codes.restype = i32

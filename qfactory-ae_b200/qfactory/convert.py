@@ -20,6 +20,8 @@ from . import layout
 def _check_weight(K, N, weight, nbits):
     assert weight.shape == (K, N), f"weight must be [K={K}, N={N}]"
     assert weight.dtype == torch.int32
+    if weight.is_cuda:
+        return   # the range is checked by the packing kernel, which reads every code anyway (_pack_native)
     lo, hi = torch.aminmax(weight)
     assert lo >= 0 and hi < 2 ** nbits, "codes out of range"
 
@@ -32,8 +34,45 @@ def _check_scale(K, N, GS, scale):
 def _check_zero(K, N, GS, zero, nbits):
     assert zero.shape == (K // GS, N)
     assert zero.dtype == torch.int32
+    if zero.is_cuda:
+        return
     lo, hi = torch.aminmax(zero)
     assert lo >= 0 and hi < 2 ** nbits, "zero-points out of range"
+
+
+def _empty_packed(K, N, nbits, GS, has_zero, dev):
+    Np = layout.padded_rows(N)
+    w = torch.empty(Np, K * nbits // 8, dtype=torch.int8, device=dev)
+    s = torch.empty(Np, K // GS, dtype=torch.float16, device=dev) if GS != -1 else None
+    z = torch.empty(Np, K // GS, dtype=torch.int8, device=dev) if has_zero else None
+    return w, s, z
+
+
+class _NoGuard:
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        return False
+
+
+_NO_GUARD = _NoGuard()
+
+
+def _on(dev):
+    """Makes `dev` current for a launch; nothing where it is already (the usual case)."""
+    return _NO_GUARD if dev.index == torch.cuda.current_device() else torch.cuda.device(dev)
+
+
+def _ptr(t):
+    return t.data_ptr() if t is not None else None
+
+
+def raise_out_of_range(flags):
+    """What the packing kernel reported (the one synchronisation of a conversion)."""
+    f = int(flags)
+    assert not f & 1, "codes out of range"
+    assert not f & 2, "zero-points out of range"
 
 
 def _pack_native(K, N, nbits, GS, weight, scale, zero, lay=layout.LAYOUT_TILE):
@@ -41,29 +80,55 @@ def _pack_native(K, N, nbits, GS, weight, scale, zero, lay=layout.LAYOUT_TILE):
 
     L = _native.lib()
     dev = weight.device
-    Np = layout.padded_rows(N)
-    w = torch.empty(Np, K * nbits // 8, dtype=torch.int8, device=dev)
-    s = z = None
-    if GS != -1:
-        s = torch.empty(Np, K // GS, dtype=torch.float16, device=dev)
-        if zero is not None:
-            z = torch.empty(Np, K // GS, dtype=torch.int8, device=dev)
+    w, s, z = _empty_packed(K, N, nbits, GS, zero is not None, dev)
     weight = weight.contiguous()
     scale_c = scale.contiguous() if scale is not None else None
     zero_c = zero.contiguous() if zero is not None else None
-    with torch.cuda.device(dev):
-        st = L.qfb_pack_layout(
-            weight.data_ptr(),
-            scale_c.data_ptr() if scale_c is not None else None,
-            zero_c.data_ptr() if zero_c is not None else None,
-            N, K, nbits, GS, lay,
-            w.data_ptr(),
-            s.data_ptr() if s is not None else None,
-            z.data_ptr() if z is not None else None,
-            torch.cuda.current_stream(dev).cuda_stream,
-        )
+    with _on(dev):
+        flags = torch.zeros(1, dtype=torch.int32, device=dev)
+        st = L.qfb_pack_checked(weight.data_ptr(), _ptr(scale_c), _ptr(zero_c), N, K, nbits, GS, lay, w.data_ptr(), _ptr(s),
+                                _ptr(z), flags.data_ptr(), torch.cuda.current_stream(dev).cuda_stream)
     _native.check(st, "qfb_pack")
+    raise_out_of_range(flags)
     return w, s, z
+
+
+def pack_gptq(K, N, nbits, GS, qweight, scale, qzeros, lay):
+    """`(w, s, z)` of `convert_params` straight from a GPTQ checkpoint's CUDA tensors: qweight int32
+    [K * nbits / 32, N], scale fp16 [K/GS, N], qzeros int32 [K/GS, >= N * nbits / 32] or None (symmetric).
+    Fields of nbits bits are always in range, so nothing is checked and nothing is waited for."""
+    from . import _native
+
+    layout.check_shape(N, K, nbits, GS)
+    _check_scale(K, N, GS, scale)
+    dev = qweight.device
+    w, s, z = _empty_packed(K, N, nbits, GS, qzeros is not None, dev)
+    qweight, scale = qweight.contiguous(), scale.contiguous()
+    qzeros = qzeros.contiguous() if qzeros is not None else None
+    with _on(dev):
+        st = _native.lib().qfb_pack_gptq(qweight.data_ptr(), scale.data_ptr(), _ptr(qzeros),
+                                         qzeros.shape[1] if qzeros is not None else 0, N, K, nbits, GS, lay, w.data_ptr(),
+                                         s.data_ptr(), _ptr(z), torch.cuda.current_stream(dev).cuda_stream)
+    _native.check(st, "qfb_pack_gptq")
+    return w, s, z
+
+
+def quantize_pack(weight, n_bits, group_size, lay):
+    """`asymmetric_quant` followed by `convert_params` of a CUDA fp16 weight [K, N], in one pass over it.  Returns
+    (w, s, z, flags): `raise_out_of_range(flags)` waits for the kernel and raises what `convert_params` raises."""
+    from . import _native
+
+    K, N = weight.shape
+    layout.check_shape(N, K, n_bits, group_size)
+    dev = weight.device
+    w, s, z = _empty_packed(K, N, n_bits, group_size, True, dev)
+    weight = weight.contiguous()
+    with _on(dev):
+        flags = torch.zeros(1, dtype=torch.int32, device=dev)
+        st = _native.lib().qfb_quantize_pack(weight.data_ptr(), N, K, n_bits, group_size, lay, w.data_ptr(), s.data_ptr(),
+                                             z.data_ptr(), flags.data_ptr(), torch.cuda.current_stream(dev).cuda_stream)
+    _native.check(st, "qfb_quantize_pack")
+    return w, s, z, flags
 
 
 def convert_params(args, params):

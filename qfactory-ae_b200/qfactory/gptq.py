@@ -66,10 +66,22 @@ def check_g_idx(g_idx: torch.Tensor, group_size: int) -> bool:
 def layer_from_gptq(qweight, qzeros, scales, bits: int, group_size: int, g_idx=None, sym: bool = False,
                     batch_size: int = 1):
     """Build a packed QLinear layer from GPTQ checkpoint tensors."""
-    from .qlinear import QLinear
+    from . import layout
+    from .convert import pack_gptq
+    from .qlinear import GPTQLinear, QLinear
 
     if g_idx is not None and not check_g_idx(g_idx, group_size):
         raise ValueError("activation-reordered GPTQ checkpoints (desc_act=True) are not supported")
+    on_gpu = qweight.is_cuda and scales.device == qweight.device and (sym or qzeros.device == qweight.device)
+    if on_gpu and bits in (2, 4, 8) and qweight.dtype == torch.int32 and group_size > 0:
+        # the packing kernel reads the checkpoint's words: no unpacked int32 copies, no range checks
+        K, N = qweight.shape[0] * (32 // bits), qweight.shape[1]
+        fits = K % group_size == 0 and (sym or (qzeros.dtype == torch.int32 and qzeros.shape[0] == K // group_size
+                                                and qzeros.shape[1] * (32 // bits) >= N))
+        if fits:
+            lay = layout.resolve_layout("auto", N, K, bits, group_size, batch_size)
+            w, s, z = pack_gptq(K, N, bits, group_size, qweight, scales.to(torch.float16), None if sym else qzeros, lay)
+            return GPTQLinear(K, N, bits, w, group_size, s, z, False, skip_convert=True, batch_size=batch_size, layout_kind=lay)
     q = unpack_qweight(qweight, bits)
     K, N = q.shape
     z = None if sym else unpack_qzeros(qzeros, bits)[:, :N].contiguous()

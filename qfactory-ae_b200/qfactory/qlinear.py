@@ -21,7 +21,7 @@ import ctypes
 import torch
 
 from . import _native, layout
-from .convert import convert_params
+from .convert import convert_params, quantize_pack, raise_out_of_range
 from .quantize import asymmetric_quant
 
 
@@ -32,20 +32,17 @@ class _PackedLinear(torch.nn.Module):
     def __init__(self, in_features, out_features, n_bits, group_size, w, s, z, max_batch=16,
                  packed_layout=layout.LAYOUT_TILE):
         super().__init__()
-        self.packed_layout = packed_layout
-        self.in_features, self.out_features = in_features, out_features
-        self.n_bits, self.group_size = n_bits, group_size
+        # plain attributes go straight into the dictionary: nn.Module's own setter looks each of them up in its tables of
+        # parameters, buffers and modules first (a third of the host time of building a layer)
+        self.__dict__.update(
+            packed_layout=packed_layout, in_features=in_features, out_features=out_features, n_bits=n_bits,
+            group_size=group_size,
+            _native_call=None,   # the C++ call object (_native.torch_module), made by _prepare
+            _flags=0, _desc=None, _ws_tensor=None, _ws_ptr=None, _ws_size=0, _max_batch=max_batch, _host=None)
         # buffers: they follow .to()/.cuda() and are saved by state_dict()
         self.register_buffer("w", w)
         self.register_buffer("s", s)
         self.register_buffer("z", z)
-        self._native_call = None   # the C++ call object (_native.torch_module), made by _prepare
-        self._flags = 0
-        self._desc = None
-        self._ws = None
-        self._ws_bytes = 0
-        self._max_batch = max_batch
-        self._host = None
 
     # -- native plumbing ---------------------------------------------------
     @property
@@ -360,5 +357,13 @@ class QLinear:
         """Quantize an fp16 weight [K, N] group-wise (asymmetric, as the reference's
         tests/acc_gptq.py:10-29 does) and pack it."""
         K, N = weight.shape
+        if weight.is_cuda and weight.dtype == torch.float16 and group_size > 0 and K % group_size == 0:
+            from . import layout as _layout
+            lay = _layout.resolve_layout(layout, N, K, n_bits, group_size, batch_size)
+            w, s, z, flags = quantize_pack(weight, n_bits, group_size, lay)
+            layer = GPTQLinear(K, N, n_bits, w, group_size, s, z, False, skip_convert=True, batch_size=batch_size,
+                               layout_kind=lay)
+            raise_out_of_range(flags)   # (the module is built while the kernel runs)
+            return layer
         q, s, z = asymmetric_quant(weight, group_size, n_bits)
         return QLinear.init(batch_size, K, N, n_bits, q, group_size, s, z, layout=layout)
