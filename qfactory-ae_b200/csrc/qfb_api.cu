@@ -233,6 +233,16 @@ static int run_tc(const LayerView& v, const __half* x, int m, __half* y, void* w
           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return QFB_ERR_CUDA;
+  CUtensorMap tw = {};
+  if (v.layout == QFB_LAYOUT_FRAGMENT && (v.bits == 4 || v.bits == 8)) {
+    const cuuint64_t wdim[2] = {16, (cuuint64_t)v.npad * v.k * v.bits / 512};
+    const cuuint64_t wstr[1] = {64};
+    const cuuint32_t wbox[2] = {16, (cuuint32_t)(16 * v.bits)};
+    if (enc(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<uint4*>(v.qw), wdim, wstr, wbox, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return QFB_ERR_CUDA;
+  }
   TcParams p = {};
   p.qw = v.qw;
   p.qs = v.qs;
@@ -285,7 +295,7 @@ static int run_tc(const LayerView& v, const __half* x, int m, __half* y, void* w
   tl_last_launch[2] = p.tail_split > 1 ? p.tail_split : grid.z;
   tl_last_launch[3] = 256 + 256 * pl.dg;
   tl_last_launch[4] = pl.nb;
-  return check_cuda(launch_gemm_tc(tm, p, v.bits, pl.nb, pl.post, pl.dg, grid, st));
+  return check_cuda(launch_gemm_tc(tm, tw, p, v.bits, pl.nb, pl.post, pl.dg, grid, st));
 }
 
 static int choose_kernel(const LayerView& v, int m, unsigned flags) {

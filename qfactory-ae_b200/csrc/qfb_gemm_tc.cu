@@ -82,6 +82,14 @@ struct TcCfg {
   static_assert(kDBase + (POST ? kRing * NB : kIssuers * NB) <= kTmemCols, "tensor memory over-subscribed");
 };
 
+// Weight stages of 4- and 8-bit fragment layers arrive through a tensor map of 64-byte rows with the 64-byte swizzle.
+// As plain bytes the 32 lanes of a decode warp read words 64 bytes apart: 4-way bank conflicts on each of the 16
+// reads, 512 shared-memory cycles a stage beside the MMAs' and the copies' own ((28672,8192) at 64 / 1024 rows 67.5
+// -> 62 and 580 -> 491 us, (8192,28672) at 128 rows 85 -> 75 us).  Not for 2 bits, whose words are 32 bytes apart
+// (2-way, and 32-byte rows would double the copy's requests), nor for 3, whose planes are read without conflicts
+// inside a row block.
+template <int BITS, bool FRAG> constexpr bool kSwizzledStage = FRAG && (BITS == 4 || BITS == 8);
+
 // ---- decode of the 64 codes thread (row, h) owns in a 128-k stage -> 32 fp16 pairs ------
 template <int BITS> struct StageDecode;
 template <> struct StageDecode<4> {
@@ -105,6 +113,8 @@ template <> struct StageDecode<4> {
 // Fragment layouts: stage = [2 halves of 64 rows][8 k-steps of 128 * BITS bytes] (qfb_common.cuh).
 // Row wt*64 + rb*16 + hh*8 + g owns, in the word frag_word_of(rb, hh) of lane g*4+t, the codes of
 // k 4t..4t+3 of a step: two exact fp16 pairs in k order per word.
+// For 4 and 8 bits the 64 bytes of a g (the words of t 0..3, 16 bytes each) arrive 64-byte-swizzled
+// (kSwizzledStage): the chunk of t sits at t ^ (g >> 1).
 template <int BITS> struct StageDecodeFragment;
 template <> struct StageDecodeFragment<4> {
   // nibbles 0,4,2,6 (hh = 0) or 1,5,3,7 (hh = 1): two LOP3 with the row's mask / magic
@@ -118,7 +128,7 @@ template <> struct StageDecodeFragment<4> {
     for (int ks = 0; ks < 4; ++ks)
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
-        const uint32_t word = *reinterpret_cast<const uint32_t*>(base + ks * 512 + t * 16);
+        const uint32_t word = *reinterpret_cast<const uint32_t*>(base + ks * 512 + ((t ^ (g >> 1)) << 4));
         d[ks * 8 + t * 2] = __hsub2(as_h2(lop3_and_or(word, mask, magic)), zs);
         d[ks * 8 + t * 2 + 1] = __hsub2(as_h2(lop3_and_or(word >> 8, mask, magic)), zs);
       }
@@ -134,7 +144,7 @@ template <> struct StageDecodeFragment<8> {
     for (int ks = 0; ks < 4; ++ks)
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
-        const uint32_t word = *reinterpret_cast<const uint32_t*>(base + ks * 1024 + t * 16);
+        const uint32_t word = *reinterpret_cast<const uint32_t*>(base + ks * 1024 + ((t ^ (g >> 1)) << 4));
         d[ks * 8 + t * 2] = __hsub2(as_h2(prmt(word, 0x64646464u, 0x4140u)), as_h2(zm.m));
         d[ks * 8 + t * 2 + 1] = __hsub2(as_h2(prmt(word, 0x64646464u, 0x4342u)), as_h2(zm.m));
       }
@@ -323,7 +333,7 @@ __device__ __forceinline__ void splitk_reduce(const float* base0, size_t sstride
 // where the scale is applied in the decode)
 template <int BITS, int NB, bool POST, int DG, bool FRAG, bool ASYM>
 __global__ void __launch_bounds__(TcCfg<BITS, NB, POST, DG>::kThreads, (TcCfg<BITS, NB, POST, DG>::kTwoPerSM ? 2 : 1))
-qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const TcParams p) {
+qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, const TcParams p) {
   using Cfg = TcCfg<BITS, NB, POST, DG>;
   constexpr int NS = Cfg::kWStages;   // weight ring
   constexpr int NX = Cfg::kXStages;   // activation ring
@@ -408,6 +418,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const TcParams p) {
     // ------------------------------ weight producer ---------------------------
     // (depends on the preceding kernel only where TcParams::early is not set: the wait above)
     if (lane == 0) {
+      if constexpr (kSwizzledStage<BITS, FRAG>) prefetch_tensormap(&tmap_w);
       const uint8_t* wsrc = reinterpret_cast<const uint8_t*>(p.qw) + ((size_t)tile * p.kblocks + kb0) * Cfg::kWBytes;
       int s = 0;
       uint32_t ph = 1;  // first pass over the ring: parity 1 of a fresh barrier passes at once
@@ -421,7 +432,12 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const TcParams p) {
         const uint32_t bar = smem_u32(&bar_wfull[s]);
         // zeros / scales of the groups this stage touches: one group, or two when the group is 64
         mbar_arrive_expect_tx(bar, Cfg::kWBytes + zb + sb + ((p.stall_test && i == 0) ? 16u : 0u));
-        if (FRAG) {
+        if constexpr (kSwizzledStage<BITS, FRAG>) {
+          // the stage is two runs: 8 k-steps (2 * BITS rows of 64 bytes each) of the upper and of the lower 64 rows
+          const int r0 = (tile * 2 * p.kblocks + kb0 + i) * (16 * BITS);
+          tma_tensor_2d_g2s(sbase + w_off + s * Cfg::kWBytes, &tmap_w, 0, r0, bar);
+          tma_tensor_2d_g2s(sbase + w_off + s * Cfg::kWBytes + Cfg::kWBytes / 2, &tmap_w, 0, r0 + p.kblocks * (16 * BITS), bar);
+        } else if (FRAG) {
           // the stage is two runs: 8 k-steps (128 * BITS bytes each) of the upper and of the lower 64 rows
           const uint8_t* f0 = reinterpret_cast<const uint8_t*>(p.qw) +
                               (((size_t)tile * 2) * (size_t)(p.kblocks * 8) + (size_t)(kb0 + i) * 8) * (128 * BITS);
@@ -668,16 +684,16 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const TcParams p) {
 // host side
 // ---------------------------------------------------------------------------------------
 template <int BITS, int NB, bool POST, int DG, bool FRAG>
-static cudaError_t launch_cfg_layout(const CUtensorMap& tm, const TcParams& p, dim3 grid, cudaStream_t st);
+static cudaError_t launch_cfg_layout(const CUtensorMap& tm, const CUtensorMap& tw, const TcParams& p, dim3 grid, cudaStream_t st);
 
 template <int BITS, int NB, bool POST, int DG>
-static cudaError_t launch_cfg(const CUtensorMap& tm, const TcParams& p, dim3 grid, cudaStream_t st) {
-  if (p.layout == QFB_LAYOUT_FRAGMENT) return launch_cfg_layout<BITS, NB, POST, DG, true>(tm, p, grid, st);
-  return launch_cfg_layout<BITS, NB, POST, DG, false>(tm, p, grid, st);
+static cudaError_t launch_cfg(const CUtensorMap& tm, const CUtensorMap& tw, const TcParams& p, dim3 grid, cudaStream_t st) {
+  if (p.layout == QFB_LAYOUT_FRAGMENT) return launch_cfg_layout<BITS, NB, POST, DG, true>(tm, tw, p, grid, st);
+  return launch_cfg_layout<BITS, NB, POST, DG, false>(tm, tw, p, grid, st);
 }
 
 template <int BITS, int NB, bool POST, int DG, bool FRAG>
-static cudaError_t launch_cfg_layout(const CUtensorMap& tm, const TcParams& p, dim3 grid, cudaStream_t st) {
+static cudaError_t launch_cfg_layout(const CUtensorMap& tm, const CUtensorMap& tw, const TcParams& p, dim3 grid, cudaStream_t st) {
   using Cfg = TcCfg<BITS, NB, POST, DG>;
   auto kern = qgemm_tc_kernel<BITS, NB, POST, DG, FRAG, false>;
   // scale-in-the-decode mode: the common case of scales and zero points present has a build of its own (measured:
@@ -698,47 +714,47 @@ static cudaError_t launch_cfg_layout(const CUtensorMap& tm, const TcParams& p, d
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, tm, p);
+  return cudaLaunchKernelEx(&cfg, kern, tm, tw, p);
 }
 
 template <int BITS, int DG>
-static cudaError_t launch_nb(const CUtensorMap& tm, const TcParams& p, int nb, bool post, dim3 grid,
+static cudaError_t launch_nb(const CUtensorMap& tm, const CUtensorMap& tw, const TcParams& p, int nb, bool post, dim3 grid,
                              cudaStream_t st) {
   if (post) {
     if (DG != 1) return cudaErrorInvalidValue;  // (narrow batch tiles: one decode group only)
     switch (nb) {
-      case 16: return launch_cfg<BITS, 16, true, 1>(tm, p, grid, st);
-      case 32: return launch_cfg<BITS, 32, true, 1>(tm, p, grid, st);
+      case 16: return launch_cfg<BITS, 16, true, 1>(tm, tw, p, grid, st);
+      case 32: return launch_cfg<BITS, 32, true, 1>(tm, tw, p, grid, st);
       default: return cudaErrorInvalidValue;
     }
   }
   switch (nb) {
-    case 64: return launch_cfg<BITS, 64, false, DG>(tm, p, grid, st);
-    case 128: return launch_cfg<BITS, 128, false, DG>(tm, p, grid, st);
-    case 256: return launch_cfg<BITS, 256, false, DG>(tm, p, grid, st);
+    case 64: return launch_cfg<BITS, 64, false, DG>(tm, tw, p, grid, st);
+    case 128: return launch_cfg<BITS, 128, false, DG>(tm, tw, p, grid, st);
+    case 256: return launch_cfg<BITS, 256, false, DG>(tm, tw, p, grid, st);
     default: return cudaErrorInvalidValue;
   }
 }
 
 template <int DG>
-static cudaError_t launch_bits(const CUtensorMap& tmap_x, const TcParams& p, int bits, int nb, bool post, dim3 grid,
+static cudaError_t launch_bits(const CUtensorMap& tmap_x, const CUtensorMap& tmap_w, const TcParams& p, int bits, int nb, bool post, dim3 grid,
                                cudaStream_t st) {
   switch (bits) {
-    case 2: return launch_nb<2, DG>(tmap_x, p, nb, post, grid, st);
-    case 3: return launch_nb<3, DG>(tmap_x, p, nb, post, grid, st);
-    case 4: return launch_nb<4, DG>(tmap_x, p, nb, post, grid, st);
-    case 8: return launch_nb<8, DG>(tmap_x, p, nb, post, grid, st);
+    case 2: return launch_nb<2, DG>(tmap_x, tmap_w, p, nb, post, grid, st);
+    case 3: return launch_nb<3, DG>(tmap_x, tmap_w, p, nb, post, grid, st);
+    case 4: return launch_nb<4, DG>(tmap_x, tmap_w, p, nb, post, grid, st);
+    case 8: return launch_nb<8, DG>(tmap_x, tmap_w, p, nb, post, grid, st);
     default: return cudaErrorInvalidValue;
   }
 }
 
-cudaError_t launch_gemm_tc(const CUtensorMap& tmap_x, const TcParams& p, int bits, int nb, bool post, int decode_groups,
+cudaError_t launch_gemm_tc(const CUtensorMap& tmap_x, const CUtensorMap& tmap_w, const TcParams& p, int bits, int nb, bool post, int decode_groups,
                            dim3 grid, cudaStream_t st) {
   // two decode groups (768 threads, one CTA per SM) where the scale is applied in the decode:
   // measured +10-17 % from 33 rows up, bit-identical results; three groups (1024 threads, 64
   // registers) were 3-6 % slower than two, and the narrow per-stage-accumulator tiles gain nothing
-  if (decode_groups == 2 && !post) return launch_bits<2>(tmap_x, p, bits, nb, post, grid, st);
-  return launch_bits<1>(tmap_x, p, bits, nb, post, grid, st);
+  if (decode_groups == 2 && !post) return launch_bits<2>(tmap_x, tmap_w, p, bits, nb, post, grid, st);
+  return launch_bits<1>(tmap_x, tmap_w, p, bits, nb, post, grid, st);
 }
 
 }  // namespace qfb

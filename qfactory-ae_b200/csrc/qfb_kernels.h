@@ -149,7 +149,9 @@ struct TcParams {
                              // that never come; every wait gives up after ~100 us (bounded-wait path under test)
 };
 // activations [m, k] fp16 row-major as a 2-D tiled tensor map with boxes of {64, nb}, 128-byte swizzle
-cudaError_t launch_gemm_tc(const CUtensorMap& tmap_x, const TcParams& p, int bits, int nb, bool post, int decode_groups,
+// tmap_w: the packed words of a 4- or 8-bit fragment layer as rows of 64 bytes, boxes of one 64-row half of a
+// 128-k stage, 64-byte swizzle (other layers: not read)
+cudaError_t launch_gemm_tc(const CUtensorMap& tmap_x, const CUtensorMap& tmap_w, const TcParams& p, int bits, int nb, bool post, int decode_groups,
                            dim3 grid, cudaStream_t st);
 
 // element-wise neighbours of the linears in a decoder layer (qfb_decoder_ops.cu)
