@@ -201,6 +201,34 @@ static size_t tc_tail_partial_bytes(const TcPlan& pl) {
   return (size_t)pl.tail_split * pl.tail_units * pl.nb * kTileRows * sizeof(float);
 }
 
+// CTA pairs (qfb_gemm_pair.cu): the batch in equal tiles of up to 256 columns, the units' K in equal runs.
+struct PairPlan { bool use; int nb, mtiles, units, pairs; bool cut; };
+
+static PairPlan plan_pair(const LayerView& v, int m) {
+  PairPlan pl = {};
+  if (m <= 128 || g_tc_nb || g_tc_split || g_tc_dg) return pl;
+  pl.mtiles = (m + 255) / 256;
+  pl.nb = ((m + pl.mtiles - 1) / pl.mtiles + 31) / 32 * 32;
+  pl.units = (v.tiles + 1) / 2 * pl.mtiles;
+  const int slots = num_sms() / 2, kblocks = v.k / 128;
+  const long long total = (long long)pl.units * kblocks;
+  // with less work per pair the single-CTA kernel's finer grid is ahead ((4096,4096): 14 stages a pair at 512 rows, 31
+  // us against 27; 28 stages at 1024 rows, 31 against 53)
+  if (total < 18LL * slots) return pl;
+  pl.use = true;
+  pl.pairs = std::min(pl.units, slots);
+  // Cutting the units costs about 20 stages of time (partial sums out and in, at the very end of the launch), so it has
+  // to save more: (4096,4096) at 1024 rows (32 stages whole, 28 cut) 40 us against 31, (12288,4096) (96, 83) 91 against
+  // 88; (8192,8192) at 256 rows (64, 28) 44 against 53, (28672,8192) at 1024 (448, 387) 375 against 394.  Runs of at
+  // least 16 stages: no run is empty, whatever its boundaries snap to.
+  const int pairs = (int)std::min<long long>(slots, total / 16);
+  if (pairs >= pl.pairs && (long long)((pl.units + slots - 1) / slots) * kblocks > total / pairs + 20) {
+    pl.pairs = pairs;
+    pl.cut = true;
+  }
+  return pl;
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -221,13 +249,14 @@ static EncodeTiledFn encode_tiled_fn() {
 
 static int run_tc(const LayerView& v, const __half* x, int m, __half* y, void* workspace, size_t ws_bytes,
                   unsigned flags, cudaStream_t st) {
-  const TcPlan pl = plan_tc(v, m);
+  const PairPlan pp = plan_pair(v, m);
+  const TcPlan pl = pp.use ? TcPlan{} : plan_tc(v, m);
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) return QFB_ERR_UNSUPPORTED;
   CUtensorMap tm;
   const cuuint64_t gdim[2] = {(cuuint64_t)v.k, (cuuint64_t)m};
   const cuuint64_t gstr[1] = {(cuuint64_t)v.k * 2};
-  const cuuint32_t box[2] = {64, (cuuint32_t)pl.nb};
+  const cuuint32_t box[2] = {64, (cuuint32_t)(pp.use ? pp.nb / 2 : pl.nb)};
   const cuuint32_t estr[2] = {1, 1};
   if (enc(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(x), gdim, gstr, box, estr,
           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -268,6 +297,29 @@ static int run_tc(const LayerView& v, const __half* x, int m, __half* y, void* w
   p.full_units = p.tail_units = 0;
   p.mtiles = pl.mtiles;
   p.stall_test = (flags & QFB_FLAG_TEST_STALLED_WAIT) ? 1 : 0;
+  if (pp.use) {
+    p.nb = pp.nb;
+    p.mtiles = pp.mtiles;
+    p.tiles = v.tiles;
+    p.units = pp.units;
+    int pairs = pp.pairs;
+    if (pp.cut) {
+      // cutting units is an optimisation: without room for the partial sums every unit runs whole
+      const size_t off = partial_offset(v.tiles);
+      if (workspace && ws_bytes >= off + pair_partial_bytes(pairs)) {
+        p.counters = reinterpret_cast<unsigned*>(static_cast<char*>(workspace) + kHeaderBytes);
+        p.partial = reinterpret_cast<float*>(static_cast<char*>(workspace) + off);
+      } else {
+        pairs = std::min(pp.units, num_sms() / 2);
+      }
+    }
+    tl_last_launch[0] = 2;
+    tl_last_launch[1] = 2 * pairs;
+    tl_last_launch[2] = p.partial ? 2 : 1;
+    tl_last_launch[3] = 768;
+    tl_last_launch[4] = pp.nb;
+    return check_cuda(launch_gemm_pair(tm, tw, p, v.bits, pairs, st));
+  }
   if (pl.split > 1) {
     const size_t off = partial_offset(v.tiles);
     const size_t need = off + (size_t)pl.split * m * v.npad * sizeof(float);
@@ -673,6 +725,8 @@ size_t qfb_workspace_bytes(int m_max, int n, int k, int bits) {
       v.group_size = gs;
       for (int m : probes) {
         if (m > m_max) continue;
+        const PairPlan pp = plan_pair(v, m);
+        if (pp.use && pp.cut) partial = std::max(partial, pair_partial_bytes(pp.pairs));
         const TcPlan pl = plan_tc(v, m);
         if (pl.split > 1) partial = std::max(partial, (size_t)pl.split * m * npad * sizeof(float));
         if (pl.tail_split > 1) partial = std::max(partial, tc_tail_partial_bytes(pl));

@@ -30,17 +30,11 @@
 #include "qfb_common.cuh"
 #include "qfb_kernels.h"
 #include "qfb_ptx.cuh"
+#include "qfb_tc_stage.cuh"
 
 namespace qfb {
 
 using namespace ptx;
-
-constexpr int kStageK = 128;              // k per pipeline stage
-constexpr int kStepsPerStage = kStageK / 16;
-constexpr int kAColsPerSlot = kStageK / 2;  // one 32-bit column holds two fp16 k
-constexpr int kDecodeWarps = 8;
-// sleep between polls of a barrier that is not ready yet, per role (ns)
-constexpr unsigned kSleepScale = 100, kSleepProducer = 100, kSleepMma = 20, kSleepDecode = 20;
 
 // DG = decode groups: 1 -> 8 decode warps (512 threads, two CTAs per SM for the smallest batch
 // tile), 2 -> two groups of 8 decode warps that take alternate stages (768 threads, one CTA per SM).
@@ -81,251 +75,6 @@ struct TcCfg {
   static_assert(kRing >= 2, "need at least two tensor-memory slots");
   static_assert(kDBase + (POST ? kRing * NB : kIssuers * NB) <= kTmemCols, "tensor memory over-subscribed");
 };
-
-// Weight stages of 4- and 8-bit fragment layers arrive through a tensor map of 64-byte rows with the 64-byte swizzle.
-// As plain bytes the 32 lanes of a decode warp read words 64 bytes apart: 4-way bank conflicts on each of the 16
-// reads, 512 shared-memory cycles a stage beside the MMAs' and the copies' own ((28672,8192) at 64 / 1024 rows 67.5
-// -> 62 and 580 -> 491 us, (8192,28672) at 128 rows 85 -> 75 us).  Not for 2 bits, whose words are 32 bytes apart
-// (2-way, and 32-byte rows would double the copy's requests), nor for 3, whose planes are read without conflicts
-// inside a row block.
-template <int BITS, bool FRAG> constexpr bool kSwizzledStage = FRAG && (BITS == 4 || BITS == 8);
-
-// ---- decode of the 64 codes thread (row, h) owns in a 128-k stage -> 32 fp16 pairs ------
-template <int BITS> struct StageDecode;
-template <> struct StageDecode<4> {
-  // stage = [4 units][128 rows][16 B]; thread owns units 2h, 2h+1
-  __device__ static __forceinline__ void run(const uint8_t* w, int row, int h, uint32_t z, __half2 (&d)[32]) {
-    const Codec<4>::ZM zm = Codec<4>::zmagic(z);
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const uint4 v = *reinterpret_cast<const uint4*>(w + (((2 * h + u) * kTileRows + row) << 4));
-      const uint32_t ww[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        __half2 t[4];
-        Codec<4>::word(ww[j], zm, t);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) d[16 * u + 4 * j + i] = t[i];
-      }
-    }
-  }
-};
-// Fragment layouts: stage = [2 halves of 64 rows][8 k-steps of 128 * BITS bytes] (qfb_common.cuh).
-// Row wt*64 + rb*16 + hh*8 + g owns, in the word frag_word_of(rb, hh) of lane g*4+t, the codes of
-// k 4t..4t+3 of a step: two exact fp16 pairs in k order per word.
-// For 4 and 8 bits the 64 bytes of a g (the words of t 0..3, 16 bytes each) arrive 64-byte-swizzled
-// (kSwizzledStage): the chunk of t sits at t ^ (g >> 1).
-template <int BITS> struct StageDecodeFragment;
-template <> struct StageDecodeFragment<4> {
-  // nibbles 0,4,2,6 (hh = 0) or 1,5,3,7 (hh = 1): two LOP3 with the row's mask / magic
-  __device__ static __forceinline__ void run(const uint8_t* w, int row, int h, uint32_t z, __half2 (&d)[32]) {
-    const Codec<4>::ZM zm = Codec<4>::zmagic(z);
-    const int wt = row >> 6, rb = (row >> 4) & 3, hh = (row >> 3) & 1, g = row & 7;
-    const uint32_t mask = hh ? 0x00f000f0u : 0x000f000fu, magic = hh ? 0x54005400u : 0x64006400u;
-    const __half2 zs = as_h2(hh ? zm.hi : zm.lo);
-    const uint8_t* base = w + wt * 4096 + (4 * h) * 512 + g * 64 + rb * 4;
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const uint32_t word = *reinterpret_cast<const uint32_t*>(base + ks * 512 + ((t ^ (g >> 1)) << 4));
-        d[ks * 8 + t * 2] = __hsub2(as_h2(lop3_and_or(word, mask, magic)), zs);
-        d[ks * 8 + t * 2 + 1] = __hsub2(as_h2(lop3_and_or(word >> 8, mask, magic)), zs);
-      }
-  }
-};
-template <> struct StageDecodeFragment<8> {
-  // one word = the row's four bytes of k 4t..4t+3
-  __device__ static __forceinline__ void run(const uint8_t* w, int row, int h, uint32_t z, __half2 (&d)[32]) {
-    const Codec<8>::ZM zm = Codec<8>::zmagic(z);
-    const int wt = row >> 6, rb = (row >> 4) & 3, hh = (row >> 3) & 1, g = row & 7;
-    const uint8_t* base = w + wt * 8192 + (4 * h) * 1024 + frag_word_offset(8, g * 4, rb * 2 + hh);
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const uint32_t word = *reinterpret_cast<const uint32_t*>(base + ks * 1024 + ((t ^ (g >> 1)) << 4));
-        d[ks * 8 + t * 2] = __hsub2(as_h2(prmt(word, 0x64646464u, 0x4140u)), as_h2(zm.m));
-        d[ks * 8 + t * 2 + 1] = __hsub2(as_h2(prmt(word, 0x64646464u, 0x4342u)), as_h2(zm.m));
-      }
-  }
-};
-template <> struct StageDecodeFragment<2> {
-  // one word = two row blocks; the row's fields sit at bit o = 4 (rb & 1) + 2 hh of each byte pair
-  __device__ static __forceinline__ void run(const uint8_t* w, int row, int h, uint32_t z, __half2 (&d)[32]) {
-    const Codec<2>::ZM zm = Codec<2>::zmagic(z);
-    const int wt = row >> 6, rb = (row >> 4) & 3, hh = (row >> 3) & 1, g = row & 7;
-    const int oi = (rb & 1) * 2 + hh;  // bit offset / 2
-    const uint32_t mask = 0x00030003u << (2 * oi);
-    const uint32_t magic = oi == 0 ? 0x64006400u : oi == 1 ? 0x5C005C00u : oi == 2 ? 0x54005400u : 0x4C004C00u;
-    const __half2 zs = as_h2(oi == 0 ? zm.m[0] : oi == 1 ? zm.m[1] : oi == 2 ? zm.m[2] : zm.m[3]);
-    const uint8_t* base = w + wt * 2048 + (4 * h) * 256 + g * 32 + (rb >> 1) * 4;
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const uint32_t word = *reinterpret_cast<const uint32_t*>(base + ks * 256 + t * 8);
-        d[ks * 8 + t * 2] = __hsub2(as_h2(lop3_and_or(word, mask, magic)), zs);
-        d[ks * 8 + t * 2 + 1] = __hsub2(as_h2(lop3_and_or(word >> 8, mask, magic)), zs);
-      }
-  }
-};
-template <> struct StageDecodeFragment<3> {
-  // word j of lane g*4+t sits in plane j (128 bytes) of the k-step (384 bytes).  Row blocks 0..2: word rb, the
-  // row's fields at bit offset 0 (rows g) or 3 (rows g + 8) for k 4t, 4t+1 and 9 bits higher for k 4t+2, 4t+3.
-  // Row block 3: offset 6 of words 0 / 1 (rows g) and of word 2 (rows g + 8, k 4t, 4t+1); rows g + 8,
-  // k 4t+2, 4t+3 are collected from the spare bits 15 / 31 of the three words.
-  __device__ static __forceinline__ void run(const uint8_t* w, int row, int h, uint32_t z, __half2 (&d)[32]) {
-    const int wt = row >> 6, rb = (row >> 4) & 3, hh = (row >> 3) & 1, g = row & 7;
-    const uint8_t* base = w + wt * 3072 + (4 * h) * 384 + g * 16;
-    if (rb < 3) {
-      // the field as the low mantissa bits of 2^(10 - offset): exact q + 2^(10 - offset), minus the same with z
-      const uint32_t mask = hh ? 0x00380038u : 0x00070007u, magic = hh ? 0x58005800u : 0x64006400u;
-      const __half2 zs = as_h2(magic | ((z << (hh ? 3 : 0)) * 0x00010001u));
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const uint32_t word = *reinterpret_cast<const uint32_t*>(base + ks * 384 + rb * 128 + t * 4);
-          d[ks * 8 + t * 2] = __hsub2(as_h2(lop3_and_or(word, mask, magic)), zs);
-          d[ks * 8 + t * 2 + 1] = __hsub2(as_h2(lop3_and_or(word >> 9, mask, magic)), zs);
-        }
-    } else {
-      const uint32_t mask = 0x01C001C0u, magic = 0x4C004C00u;
-      const __half2 zs = as_h2(magic | ((z << 6) * 0x00010001u));
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const uint8_t* p = base + ks * 384 + t * 4;
-          const uint32_t w0 = *reinterpret_cast<const uint32_t*>(p), w1 = *reinterpret_cast<const uint32_t*>(p + 128),
-                         w2 = *reinterpret_cast<const uint32_t*>(p + 256);
-          const uint32_t spare = ((w0 >> 9) & 0x00400040u) | ((w1 >> 8) & 0x00800080u) | ((w2 >> 7) & 0x01000100u);
-          const uint32_t lo = hh ? (w2 & mask) : (w0 & mask), hi = hh ? spare : (w1 & mask);
-          d[ks * 8 + t * 2] = __hsub2(as_h2(lo | magic), zs);
-          d[ks * 8 + t * 2 + 1] = __hsub2(as_h2(hi | magic), zs);
-        }
-    }
-  }
-};
-template <> struct StageDecode<8> {
-  // stage = [8 units][128 rows][16 B]; thread owns units 4h .. 4h+3
-  __device__ static __forceinline__ void run(const uint8_t* w, int row, int h, uint32_t z, __half2 (&d)[32]) {
-    const Codec<8>::ZM zm = Codec<8>::zmagic(z);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const uint4 v = *reinterpret_cast<const uint4*>(w + (((4 * h + u) * kTileRows + row) << 4));
-      const uint32_t ww[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        d[8 * u + 2 * j] = __hsub2(as_h2(prmt(ww[j], 0x64646464u, 0x4140u)), as_h2(zm.m));
-        d[8 * u + 2 * j + 1] = __hsub2(as_h2(prmt(ww[j], 0x64646464u, 0x4342u)), as_h2(zm.m));
-      }
-    }
-  }
-};
-template <> struct StageDecode<2> {
-  // stage = [2 units][128 rows][16 B]; thread owns unit h
-  __device__ static __forceinline__ void run(const uint8_t* w, int row, int h, uint32_t z, __half2 (&d)[32]) {
-    const uint4 v = *reinterpret_cast<const uint4*>(w + ((h * kTileRows + row) << 4));
-    const Codec<2>::ZM zm = Codec<2>::zmagic(z);
-    const uint32_t ww[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      __half2 t[4];
-      Codec<2>::half_word(ww[j], zm, t);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) d[8 * j + i] = t[i];
-      Codec<2>::half_word(ww[j] >> 8, zm, t);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) d[8 * j + 4 + i] = t[i];
-    }
-  }
-};
-template <> struct StageDecode<3> {
-  // stage = one 3-bit unit = [3 vectors][128 rows][16 B]: two 2-bit-plane vectors and the
-  // 1-bit-plane vector; thread owns 2-bit vector h and words 2h, 2h+1 of the plane vector
-  __device__ static __forceinline__ void run(const uint8_t* w, int row, int h, uint32_t z, __half2 (&d)[32]) {
-    const uint4 a = *reinterpret_cast<const uint4*>(w + ((h * kTileRows + row) << 4));
-    const uint2 b = *reinterpret_cast<const uint2*>(w + ((2 * kTileRows + row) << 4) + (h << 3));
-    const Codec<3>::ZM zm = Codec<3>::zmagic(z);
-    const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
-    const uint32_t bw[2] = {b.x, b.y};
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {  // 32 codes: 2-bit words aw[2j], aw[2j+1] with plane word bw[j]
-      __half2 t[4];
-      Codec<3>::half_word(aw[2 * j], bw[j] << 2, zm, t);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) d[16 * j + i] = t[i];
-      Codec<3>::half_word(aw[2 * j] >> 8, bw[j] << 1, zm, t);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) d[16 * j + 4 + i] = t[i];
-      Codec<3>::half_word(aw[2 * j + 1], bw[j] >> 6, zm, t);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) d[16 * j + 8 + i] = t[i];
-      Codec<3>::half_word(aw[2 * j + 1] >> 8, bw[j] >> 7, zm, t);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) d[16 * j + 12 + i] = t[i];
-    }
-  }
-};
-
-// Sum of the split-K partials of one warp's 32 rows (lane = row) over all S splits, in split order,
-// rounded to fp16 into y.  base0 -> partial of split 0, batch column 0, this lane's row; `sstride`
-// floats between splits, `cstride` between batch columns; ydst -> y[first batch row][this lane's
-// output feature], `ystride` halfs between batch rows; `cols` = valid batch columns.
-// Loads in flight per round: 32 batch columns of one split where one accumulator spans K (this
-// warp's own sums, the same bits it published, are re-read from tensor memory at taddr_own instead,
-// plus the second issuer's accumulator when `two`); 8 columns of four splits for the narrow
-// per-stage-accumulator tiles, which have many splits.  (A column at a time cost one round trip per
-// column: the reduce of a wide tile then took longer than its MMAs.  Measured against 16 columns of
-// two splits and against a non-inlined function: this form is 2-7 % faster on every batch size.)
-template <int NB, bool POST>
-__device__ __forceinline__ void splitk_reduce(const float* base0, size_t sstride, size_t cstride, int S, int split, int cols,
-                                           bool row_ok, __half* ydst, size_t ystride, uint32_t taddr_own, bool two) {
-  constexpr int CW = POST ? 8 : 32, SPB = POST ? 4 : 1;
-#pragma unroll 1
-  for (int c0 = 0; c0 < NB; c0 += CW) {
-    if (c0 >= cols) break;
-    float sum[CW];
-#pragma unroll
-    for (int j = 0; j < CW; ++j) sum[j] = 0.f;
-#pragma unroll 1
-    for (int sp = 0; sp < S; sp += SPB) {
-      float t[SPB][CW];
-#pragma unroll
-      for (int u = 0; u < SPB; ++u) {
-        if (!POST && sp + u == split) continue;   // filled below, without a load
-#pragma unroll
-        for (int j = 0; j < CW; ++j)
-          t[u][j] = (sp + u < S && c0 + j < cols) ? __ldcg(base0 + (size_t)(sp + u) * sstride + (size_t)(c0 + j) * cstride) : 0.f;
-      }
-      if (!POST) {
-#pragma unroll
-        for (int u = 0; u < SPB; ++u)
-          if (sp + u == split) {
-#pragma unroll
-            for (int c = 0; c < CW; c += 16) {
-              uint32_t v[16], v2[16];
-              tmem_ld_x16(taddr_own + c0 + c, v);
-              if (two) tmem_ld_x16(taddr_own + NB + c0 + c, v2);
-              tmem_wait_ld();
-#pragma unroll
-              for (int j = 0; j < 16; ++j) t[u][c + j] = __uint_as_float(v[j]) + (two ? __uint_as_float(v2[j]) : 0.f);
-            }
-          }
-      }
-#pragma unroll
-      for (int u = 0; u < SPB; ++u)
-#pragma unroll
-        for (int j = 0; j < CW; ++j)
-          if (sp + u < S) sum[j] += t[u][j];
-    }
-#pragma unroll
-    for (int j = 0; j < CW; ++j)
-      if (c0 + j < cols && row_ok) ydst[(size_t)(c0 + j) * ystride] = __float2half_rn(sum[j]);
-  }
-}
 
 // FRAG = the layer is in the fragment layout (a build of its own: with both decoders behind a run-time branch in
 // the decode loop the compiler allots registers for the larger of the two)

@@ -147,12 +147,22 @@ struct TcParams {
   int mtiles;                // batch tiles per row tile (unit = tile * mtiles + batch tile)
   int stall_test;            // 1 (QFB_FLAG_TEST_STALLED_WAIT): the first weight stage's barrier expects 16 bytes
                              // that never come; every wait gives up after ~100 us (bounded-wait path under test)
+  // CTA pairs (launch_gemm_pair):
+  int nb;                    // columns of a batch tile, a multiple of 32 up to 256
+  int tiles;                 // row tiles of the layer
+  int units;                 // (pair of row tiles, batch tile) units; unit = pair of tiles * mtiles + batch tile
 };
 // activations [m, k] fp16 row-major as a 2-D tiled tensor map with boxes of {64, nb}, 128-byte swizzle
 // tmap_w: the packed words of a 4- or 8-bit fragment layer as rows of 64 bytes, boxes of one 64-row half of a
 // 128-k stage, 64-byte swizzle (other layers: not read)
 cudaError_t launch_gemm_tc(const CUtensorMap& tmap_x, const CUtensorMap& tmap_w, const TcParams& p, int bits, int nb, bool post, int decode_groups,
                            dim3 grid, cudaStream_t st);
+
+// the same product on `pairs` persistent CTA pairs (qfb_gemm_pair.cu); tmap_x with boxes of {64, p.nb / 2}.
+// p.partial null: units are not cut; else room for pair_partial_bytes, and p.counters has 8 words per pair.
+cudaError_t launch_gemm_pair(const CUtensorMap& tmap_x, const CUtensorMap& tmap_w, const TcParams& p, int bits, int pairs,
+                             cudaStream_t st);
+inline size_t pair_partial_bytes(int pairs) { return (size_t)pairs * 4 * 256 * 128 * sizeof(float); }
 
 // element-wise neighbours of the linears in a decoder layer (qfb_decoder_ops.cu)
 cudaError_t launch_rmsnorm(__half* x, const __half* res, const __half* w, __half* y, int rows, int d, float eps,

@@ -82,6 +82,71 @@ __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
 }
 
+// ---- CTA pairs ---------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// this CTA's shared-memory address in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// Relaxed: what these arrivals publish is in tensor memory, ordered by tcgen05.wait and tcgen05.fence around them.  (A
+// release at cluster scope waited for the warp's other memory operations on every stage: (28672,8192) at 1024 rows
+// 449 us instead of 385.)
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// a barrier on which threads of both CTAs arrive with mbar_arrive_cluster
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "r"(kSuspendHintNs)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+                                                  unsigned backoff_ns, long long limit_cycles) {
+  if (mbar_try_wait_cluster(bar, parity)) return true;
+  const long long t0 = clock64();
+  int it = 0;
+  while (!mbar_try_wait_cluster(bar, parity)) {
+    if (backoff_ns) __nanosleep(backoff_ns);
+    if ((++it & 15) == 0) {
+      if (*abort_flag) return false;
+      if (clock64() - t0 > limit_cycles) {
+        *abort_flag = 1;
+        return false;
+      }
+    }
+  }
+  return true;
+}
+// into this CTA's shared memory, counted on a barrier of either CTA of the pair (`bar`: shared::cluster address)
+__device__ __forceinline__ void tma_tensor_2d_g2s_pair(uint32_t dst, const CUtensorMap* tmap, int c0, int c1, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+      "l"(tmap), "r"(c0), "r"(c1), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+
 // ---- tensor memory -----------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols) : "memory");
@@ -129,38 +194,54 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uin
 // The eight k16 steps of one 128-k stage in a single block: A advances 8 columns per step,
 // B walks two 128-byte-swizzled 64-k atoms (descriptor low words b0_lo / b1_lo, +32 bytes per
 // step).  `first_accumulates` = 0 makes step 0 overwrite D.
+#define QFB_MMA_STAGE8(CG) \
+  asm volatile( \
+      "{\n\t" \
+      ".reg .pred p0, p1;\n\t" \
+      ".reg .b64 bd;\n\t" \
+      ".reg .b32 a, bl;\n\t" \
+      "setp.ne.b32 p0, %6, 0;\n\t" \
+      "setp.eq.b32 p1, 0, 0;\n\t" \
+      "mov.b64 bd, {%2, %4};\n\t" \
+      "tcgen05.mma.cta_group::" CG ".kind::f16 [%0], [%1], bd, %5, p0;\n\t" \
+      "add.u32 a, %1, 8;\n\t  add.u32 bl, %2, 2;\n\t  mov.b64 bd, {bl, %4};\n\t" \
+      "tcgen05.mma.cta_group::" CG ".kind::f16 [%0], [a], bd, %5, p1;\n\t" \
+      "add.u32 a, %1, 16;\n\t add.u32 bl, %2, 4;\n\t  mov.b64 bd, {bl, %4};\n\t" \
+      "tcgen05.mma.cta_group::" CG ".kind::f16 [%0], [a], bd, %5, p1;\n\t" \
+      "add.u32 a, %1, 24;\n\t add.u32 bl, %2, 6;\n\t  mov.b64 bd, {bl, %4};\n\t" \
+      "tcgen05.mma.cta_group::" CG ".kind::f16 [%0], [a], bd, %5, p1;\n\t" \
+      "add.u32 a, %1, 32;\n\t mov.b64 bd, {%3, %4};\n\t" \
+      "tcgen05.mma.cta_group::" CG ".kind::f16 [%0], [a], bd, %5, p1;\n\t" \
+      "add.u32 a, %1, 40;\n\t add.u32 bl, %3, 2;\n\t  mov.b64 bd, {bl, %4};\n\t" \
+      "tcgen05.mma.cta_group::" CG ".kind::f16 [%0], [a], bd, %5, p1;\n\t" \
+      "add.u32 a, %1, 48;\n\t add.u32 bl, %3, 4;\n\t  mov.b64 bd, {bl, %4};\n\t" \
+      "tcgen05.mma.cta_group::" CG ".kind::f16 [%0], [a], bd, %5, p1;\n\t" \
+      "add.u32 a, %1, 56;\n\t add.u32 bl, %3, 6;\n\t  mov.b64 bd, {bl, %4};\n\t" \
+      "tcgen05.mma.cta_group::" CG ".kind::f16 [%0], [a], bd, %5, p1;\n\t" \
+      "}" ::"r"(d_tmem), \
+      "r"(a_tmem), "r"(b0_lo), "r"(b1_lo), "r"(b_hi), "r"(idesc), "r"(first_accumulates) \
+      : "memory")
 __device__ __forceinline__ void mma_f16_ts_stage8(uint32_t d_tmem, uint32_t a_tmem, uint32_t b0_lo, uint32_t b1_lo,
                                                   uint32_t b_hi, uint32_t idesc, uint32_t first_accumulates) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p0, p1;\n\t"
-      ".reg .b64 bd;\n\t"
-      ".reg .b32 a, bl;\n\t"
-      "setp.ne.b32 p0, %6, 0;\n\t"
-      "setp.eq.b32 p1, 0, 0;\n\t"
-      "mov.b64 bd, {%2, %4};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %5, p0;\n\t"
-      "add.u32 a, %1, 8;\n\t  add.u32 bl, %2, 2;\n\t  mov.b64 bd, {bl, %4};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], bd, %5, p1;\n\t"
-      "add.u32 a, %1, 16;\n\t add.u32 bl, %2, 4;\n\t  mov.b64 bd, {bl, %4};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], bd, %5, p1;\n\t"
-      "add.u32 a, %1, 24;\n\t add.u32 bl, %2, 6;\n\t  mov.b64 bd, {bl, %4};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], bd, %5, p1;\n\t"
-      "add.u32 a, %1, 32;\n\t mov.b64 bd, {%3, %4};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], bd, %5, p1;\n\t"
-      "add.u32 a, %1, 40;\n\t add.u32 bl, %3, 2;\n\t  mov.b64 bd, {bl, %4};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], bd, %5, p1;\n\t"
-      "add.u32 a, %1, 48;\n\t add.u32 bl, %3, 4;\n\t  mov.b64 bd, {bl, %4};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], bd, %5, p1;\n\t"
-      "add.u32 a, %1, 56;\n\t add.u32 bl, %3, 6;\n\t  mov.b64 bd, {bl, %4};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], bd, %5, p1;\n\t"
-      "}" ::"r"(d_tmem),
-      "r"(a_tmem), "r"(b0_lo), "r"(b1_lo), "r"(b_hi), "r"(idesc), "r"(first_accumulates)
-      : "memory");
+  QFB_MMA_STAGE8("1");
 }
+// the same for a CTA pair: 256 rows of A (128 in each CTA's tensor memory), each CTA's half of B in its shared memory
+__device__ __forceinline__ void mma_f16_ts_stage8_pair(uint32_t d_tmem, uint32_t a_tmem, uint32_t b0_lo, uint32_t b1_lo,
+                                                       uint32_t b_hi, uint32_t idesc, uint32_t first_accumulates) {
+  QFB_MMA_STAGE8("2");
+}
+#undef QFB_MMA_STAGE8
 // arrive on an mbarrier once every tcgen05 operation issued so far by this thread is done
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+// the same from a CTA pair's MMAs, on the barrier at this offset in both CTAs
+__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .b16 mask;\n\tmov.b16 mask, 3;\n\t"
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], mask;\n\t}" ::"r"(bar)
+      : "memory");
 }
 
 // K-major, 128-byte-swizzled shared-memory operand descriptor (8-row groups 1024 bytes apart)
@@ -172,6 +253,10 @@ __device__ __forceinline__ uint64_t smem_desc_k_sw128(uint32_t saddr) {
   d |= (uint64_t)1 << 46;                          // descriptor version (Blackwell)
   d |= (uint64_t)2 << 61;                          // layout type: SWIZZLE_128B
   return d;
+}
+// fp16 x fp16 -> fp32, both operands K-major, M = 256 over a CTA pair
+__host__ __device__ constexpr uint32_t idesc_f16_m256(int n) {
+  return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
 }
 // fp16 x fp16 -> fp32, both operands K-major, M = 128
 __host__ __device__ constexpr uint32_t idesc_f16_m128(int n) {
