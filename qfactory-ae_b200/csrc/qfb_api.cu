@@ -121,7 +121,11 @@ static size_t partial_offset(int tiles) { return kHeaderBytes + counters_bytes(t
 // ---- tensor-core path planning --------------------------------------------------------
 struct TcPlan { int nb, mtiles, split, dg; bool post; int tail_split, full_units, tail_units; };
 
-static bool tc_supported(const LayerView& v) { return v.k % 128 == 0; }
+// A 128-k stage lies in one quantisation group or holds two groups of 64: other odd multiples of 64 (192, 320) straddle
+// stages and are served by the CUDA-core kernel.
+static bool tc_supported(const LayerView& v) {
+  return v.k % 128 == 0 && (v.group_size == -1 || v.group_size == 64 || v.group_size % 128 == 0);
+}
 
 static TcPlan plan_tc(const LayerView& v, int m) {
   TcPlan pl;
