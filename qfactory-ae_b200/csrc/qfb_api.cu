@@ -121,10 +121,12 @@ static size_t partial_offset(int tiles) { return kHeaderBytes + counters_bytes(t
 // ---- tensor-core path planning --------------------------------------------------------
 struct TcPlan { int nb, mtiles, split, dg; bool post; int tail_split, full_units, tail_units; };
 
+static int stages_of(const LayerView& v) { return (v.k + 127) / 128; }
+
 // A 128-k stage lies in one quantisation group or holds two groups of 64: other odd multiples of 64 (192, 320) straddle
 // stages and are served by the CUDA-core kernel.
 static bool tc_supported(const LayerView& v) {
-  return v.k % 128 == 0 && (v.group_size == -1 || v.group_size == 64 || v.group_size % 128 == 0);
+  return v.group_size == -1 || v.group_size == 64 || v.group_size % 128 == 0;
 }
 
 static TcPlan plan_tc(const LayerView& v, int m) {
@@ -140,7 +142,7 @@ static TcPlan plan_tc(const LayerView& v, int m) {
     pl.post = post_ok && m <= 32;
     pl.nb = !pl.post ? 64 : m <= 16 ? 16 : 32;
     pl.mtiles = 1;
-    const int kblocks = v.k / 128;
+    const int kblocks = stages_of(v);
     const int target = num_sms() * ((pl.post && pl.nb <= 32 && pl.dg == 1) ? 2 : 1);
     int split = std::max(1, target / v.tiles);
     split = std::min(split, std::max(1, kblocks / 4));
@@ -152,7 +154,7 @@ static TcPlan plan_tc(const LayerView& v, int m) {
       if (v.tiles >= 90) split = 1;
       else while (split & (split - 1)) split &= split - 1;
     }
-    if (pl.nb == 64 && kblocks < 160) split = 1;
+    if (pl.nb == 64 && kblocks < 160 && v.tiles > num_sms() / 3) split = 1;
     if (g_tc_split > 0) split = std::min(g_tc_split, std::max(1, kblocks));
     if (v.tiles > 512) split = 1;  // the counter array holds 512 tiles x 4 row quarters
     pl.split = split;
@@ -167,7 +169,7 @@ static TcPlan plan_tc(const LayerView& v, int m) {
     if (pl.nb == 64 && (long long)v.tiles * ((m + 127) / 128) >= num_sms() / 2) pl.nb = 128;
     if (g_tc_nb == 64 || g_tc_nb == 128 || g_tc_nb == 256) pl.nb = g_tc_nb;
     pl.mtiles = (m + pl.nb - 1) / pl.nb;
-    const int kblocks = v.k / 128;
+    const int kblocks = stages_of(v);
     if (g_tc_split > 1) {  // tuning override: every unit is cut
       pl.tail_split = std::min(g_tc_split, 4);
     } else if (g_tc_split == 0 && g_tc_nb == 0 && m >= 96 && m <= 512 && kblocks >= 64) {
@@ -214,7 +216,7 @@ static PairPlan plan_pair(const LayerView& v, int m) {
   pl.mtiles = (m + 255) / 256;
   pl.nb = ((m + pl.mtiles - 1) / pl.mtiles + 31) / 32 * 32;
   pl.units = (v.tiles + 1) / 2 * pl.mtiles;
-  const int slots = num_sms() / 2, kblocks = v.k / 128;
+  const int slots = num_sms() / 2, kblocks = stages_of(v);
   const long long total = (long long)pl.units * kblocks;
   // with less work per pair the single-CTA kernel's finer grid is ahead ((4096,4096): 14 stages a pair at 512 rows, 31
   // us against 27; 28 stages at 1024 rows, 31 against 53)
@@ -286,7 +288,8 @@ static int run_tc(const LayerView& v, const __half* x, int m, __half* y, void* w
   p.k = v.k;
   p.npad = v.npad;
   p.groups = v.groups;
-  p.kblocks = v.k / 128;
+  p.kblocks = stages_of(v);
+  p.half_tail = v.k % 128 != 0;
   const int gs = v.group_size == -1 ? v.k : v.group_size;
   p.steps_per_group = gs / 16;
   p.halfstages_per_group = gs / 64;
@@ -324,14 +327,20 @@ static int run_tc(const LayerView& v, const __half* x, int m, __half* y, void* w
     tl_last_launch[4] = pp.nb;
     return check_cuda(launch_gemm_pair(tm, tw, p, v.bits, pairs, st));
   }
-  if (pl.split > 1) {
+  int split = pl.split;
+  if (split > 1) {
     const size_t off = partial_offset(v.tiles);
-    const size_t need = off + (size_t)pl.split * m * v.npad * sizeof(float);
-    if (!workspace || ws_bytes < need) return QFB_ERR_WORKSPACE;
-    p.counters = reinterpret_cast<unsigned*>(static_cast<char*>(workspace) + kHeaderBytes);
-    p.partial = reinterpret_cast<float*>(static_cast<char*>(workspace) + off);
+    const size_t need = off + (size_t)split * m * v.npad * sizeof(float);
+    if (workspace && ws_bytes >= need) {
+      p.counters = reinterpret_cast<unsigned*>(static_cast<char*>(workspace) + kHeaderBytes);
+      p.partial = reinterpret_cast<float*>(static_cast<char*>(workspace) + off);
+    } else if (v.k % 128 == 0) {
+      return QFB_ERR_WORKSPACE;
+    } else {
+      split = 1;   // (these sizes also run with the smaller workspace of the CUDA-core kernel)
+    }
   }
-  dim3 grid(v.tiles, pl.mtiles, pl.split);
+  dim3 grid(v.tiles, pl.mtiles, split);
   if (pl.tail_split > 1) {
     // the tail split is an optimisation: a workspace too small for its partial sums means the
     // plain grid, not an error (the counters of tail units sit in the first 2048 slots)
@@ -357,6 +366,9 @@ static int run_tc(const LayerView& v, const __half* x, int m, __half* y, void* w
 static int choose_kernel(const LayerView& v, int m, unsigned flags) {
   if (flags & QFB_FLAG_FORCE_SIMT) return 1;
   if (!tc_supported(v)) return 1;
+  // K an odd multiple of 64: the CUDA-core kernel takes 8 rows a pass and reads the weights again for every 8 more
+  // ((3000,2752) at 37 rows: 79 us against 20)
+  if (v.k % 128 != 0) return m > kMaxSimtRows ? 2 : 1;
   if (flags & QFB_FLAG_FORCE_TENSOR) return 2;
   if (m >= g_tc_min_m) return 2;
   // a single activation row: the CUDA-core kernel wins while the packed weight is small
@@ -721,7 +733,7 @@ size_t qfb_workspace_bytes(int m_max, int n, int k, int bits) {
   const int tiles = npad / kTileRows;
   const int rows = std::min(m_max, kMaxSimtRows);
   size_t partial = (size_t)split_cap(tiles, k / unit_k(bits)) * rows * npad * sizeof(float);
-  if (k % 128 == 0) {
+  {
     LayerView v = {};
     v.n = n; v.k = k; v.bits = bits; v.npad = npad; v.tiles = tiles;
     const int probes[] = {16, 32, 64, 96, 128, 192, 256, 384, 512, 768, 1024, 1536, 2048, 4096, m_max};

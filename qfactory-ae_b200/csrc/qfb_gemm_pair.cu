@@ -313,7 +313,11 @@ qgemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         for (int i = 0; i < j.nkb; ++i) {
           if (!mbar_wait(smem_u32(&bar_wempty[s]), ph, abortp, kSleepProducer, wait_limit)) { ok = false; break; }
           const uint32_t bar = smem_u32(&bar_wfull[s]);
-          mbar_arrive_expect_tx(bar, Cfg::kWBytes + zb + sb + ((p.stall_test && at == s_begin + j.nkb && i == 0) ? 16u : 0u));
+          // (K an odd multiple of 64: the last stage is half a stage of codes, and one group of 64)
+          const bool half = !FRAG && p.half_tail && j.kb0 + i == p.kblocks - 1;
+          const uint32_t wb = half ? Cfg::kWBytes / 2 : Cfg::kWBytes;
+          const uint32_t zn = half && hpg == 1 ? zb / 2 : zb, sn = half && hpg == 1 ? sb / 2 : sb;
+          mbar_arrive_expect_tx(bar, wb + zn + sn + ((p.stall_test && at == s_begin + j.nkb && i == 0) ? 16u : 0u));
           const uint32_t dst = sbase + w_off + s * Cfg::kWBytes;
           if constexpr (kSwizzledStage<BITS, FRAG>) {
             const int r0 = (tile * 2 * p.kblocks + j.kb0 + i) * (16 * BITS);
@@ -325,11 +329,11 @@ qgemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             tma_bulk_g2s(dst, f0, Cfg::kWBytes / 2, bar);
             tma_bulk_g2s(dst + Cfg::kWBytes / 2, f0 + (size_t)p.kblocks * 8 * (128 * BITS), Cfg::kWBytes / 2, bar);
           } else {
-            tma_bulk_g2s(dst, reinterpret_cast<const uint8_t*>(p.qw) + ((size_t)tile * p.kblocks + j.kb0 + i) * Cfg::kWBytes,
-                         Cfg::kWBytes, bar);
+            tma_bulk_g2s(dst, reinterpret_cast<const uint8_t*>(p.qw) + (size_t)tile * p.k * (16 * BITS) +
+                                  (size_t)(j.kb0 + i) * Cfg::kWBytes, wb, bar);
           }
-          if (zb) tma_bulk_g2s(sbase + z_off + s * Cfg::kZSlot, p.qz + ((size_t)tile * p.groups + g0) * kTileRows, zb, bar);
-          if (sb) tma_bulk_g2s(sbase + s_off + s * Cfg::kSSlot, p.qs + ((size_t)tile * p.groups + g0) * kTileRows, sb, bar);
+          if (zn) tma_bulk_g2s(sbase + z_off + s * Cfg::kZSlot, p.qz + ((size_t)tile * p.groups + g0) * kTileRows, zn, bar);
+          if (sn) tma_bulk_g2s(sbase + s_off + s * Cfg::kSSlot, p.qs + ((size_t)tile * p.groups + g0) * kTileRows, sn, bar);
           gpos += 2;
           if (hpg == 1) { g0 += 2; gpos = 0; } else if (gpos >= hpg) { gpos = 0; ++g0; }
           if (++s == NS) { s = 0; ph ^= 1; }
@@ -408,7 +412,7 @@ qgemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     const int qsel = (p.halfstages_per_group == 1 && h == 1) ? kTileRows : 0;
     const int qrow = qsel + (FRAG ? frag_pos_of_row(row) : row);
     const uint32_t afull0 = mapa(smem_u32(&bar_afull[0]), 0);
-    const int n_stages = (int)(s_end - s_begin);
+    const int n_stages = (int)(s_end - s_begin), kb_first = (int)(s_begin % p.kblocks);
     for (int i = grp; i < n_stages; i += DG) {
       const int s = i % NS, r = i % R;
       if (!mbar_wait(smem_u32(&bar_wfull[s]), (uint32_t)(i / NS) & 1u, abortp, kSleepDecode, wait_limit)) break;
@@ -424,6 +428,11 @@ qgemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       } else {
 #pragma unroll
         for (int j = 0; j < 32; ++j) rr[j] = as_u32(d[j]);
+      }
+      // the upper half of a half-filled last stage: its activations are zero-filled, its slot holds older bytes
+      if (!FRAG && p.half_tail && h == 1 && (kb_first + i) % p.kblocks == p.kblocks - 1) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) rr[j] = 0u;
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&bar_wempty[s]));

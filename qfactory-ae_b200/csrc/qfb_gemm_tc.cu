@@ -168,7 +168,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
     // (depends on the preceding kernel only where TcParams::early is not set: the wait above)
     if (lane == 0) {
       if constexpr (kSwizzledStage<BITS, FRAG>) prefetch_tensormap(&tmap_w);
-      const uint8_t* wsrc = reinterpret_cast<const uint8_t*>(p.qw) + ((size_t)tile * p.kblocks + kb0) * Cfg::kWBytes;
+      const uint8_t* wsrc = reinterpret_cast<const uint8_t*>(p.qw) + (size_t)tile * p.k * (16 * BITS) + (size_t)kb0 * Cfg::kWBytes;
       int s = 0;
       uint32_t ph = 1;  // first pass over the ring: parity 1 of a fresh barrier passes at once
       // group of the stage's first 64 k, tracked without divisions in the loop
@@ -179,8 +179,12 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
       for (int i = 0; i < nkb; ++i) {
         if (!mbar_wait(smem_u32(&bar_wempty[s]), ph, abortp, kSleepProducer, wait_limit)) break;
         const uint32_t bar = smem_u32(&bar_wfull[s]);
+        // (K an odd multiple of 64: the last stage is half a stage of codes, and one group of 64)
+        const bool half = !FRAG && p.half_tail && kb0 + i == p.kblocks - 1;
+        const uint32_t wb = half ? Cfg::kWBytes / 2 : Cfg::kWBytes;
+        const uint32_t zn = half && hpg == 1 ? zb / 2 : zb, sn = half && hpg == 1 ? sb / 2 : sb;
         // zeros / scales of the groups this stage touches: one group, or two when the group is 64
-        mbar_arrive_expect_tx(bar, Cfg::kWBytes + zb + sb + ((p.stall_test && i == 0) ? 16u : 0u));
+        mbar_arrive_expect_tx(bar, wb + zn + sn + ((p.stall_test && i == 0) ? 16u : 0u));
         if constexpr (kSwizzledStage<BITS, FRAG>) {
           // the stage is two runs: 8 k-steps (2 * BITS rows of 64 bytes each) of the upper and of the lower 64 rows
           const int r0 = (tile * 2 * p.kblocks + kb0 + i) * (16 * BITS);
@@ -194,10 +198,10 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
           tma_bulk_g2s(sbase + w_off + s * Cfg::kWBytes + Cfg::kWBytes / 2,
                        f0 + (size_t)p.kblocks * 8 * (128 * BITS), Cfg::kWBytes / 2, bar);
         } else {
-          tma_bulk_g2s(sbase + w_off + s * Cfg::kWBytes, wsrc + (size_t)i * Cfg::kWBytes, Cfg::kWBytes, bar);
+          tma_bulk_g2s(sbase + w_off + s * Cfg::kWBytes, wsrc + (size_t)i * Cfg::kWBytes, wb, bar);
         }
-        if (zb) tma_bulk_g2s(sbase + z_off + s * Cfg::kZSlot, p.qz + ((size_t)tile * p.groups + g0) * kTileRows, zb, bar);
-        if (sb) tma_bulk_g2s(sbase + s_off + s * Cfg::kSSlot, p.qs + ((size_t)tile * p.groups + g0) * kTileRows, sb, bar);
+        if (zn) tma_bulk_g2s(sbase + z_off + s * Cfg::kZSlot, p.qz + ((size_t)tile * p.groups + g0) * kTileRows, zn, bar);
+        if (sn) tma_bulk_g2s(sbase + s_off + s * Cfg::kSSlot, p.qs + ((size_t)tile * p.groups + g0) * kTileRows, sn, bar);
         gpos += 2;
         if (hpg == 1) { g0 += 2; gpos = 0; } else if (gpos >= hpg) { gpos = 0; ++g0; }
         if (++s == NS) { s = 0; ph ^= 1; }
@@ -280,6 +284,11 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
       } else {
 #pragma unroll
         for (int j = 0; j < 32; ++j) rr[j] = as_u32(d[j]);
+      }
+      // the upper half of a half-filled last stage: its activations are zero-filled, its slot holds older bytes
+      if (!FRAG && p.half_tail && h == 1 && kb0 + i == p.kblocks - 1) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) rr[j] = 0u;
       }
       // the packed stage is in registers: hand the shared-memory slot back to the producer
       __syncwarp();

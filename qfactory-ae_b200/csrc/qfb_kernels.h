@@ -134,7 +134,8 @@ struct TcParams {
   unsigned* status;      // set to 1 when a bounded wait ran out
   int m, n, k, npad;
   int groups;
-  int kblocks;               // K / 128 pipeline stages
+  int kblocks;               // pipeline stages of 128 k
+  int half_tail;             // K is an odd multiple of 64 (tile layout): the last stage holds 64 k
   int steps_per_group;       // group_size / 16 MMA k-steps per quantisation group (K / 16 when group-less)
   int halfstages_per_group;  // group_size / 64
   uint32_t zconst;
