@@ -154,7 +154,10 @@ static TcPlan plan_tc(const LayerView& v, int m) {
       if (v.tiles >= 90) split = 1;
       else while (split & (split - 1)) split &= split - 1;
     }
-    if (pl.nb == 64 && kblocks < 160 && v.tiles > num_sms() / 3) split = 1;
+    // one accumulator over K: a split saves half a microsecond a stage and costs about three in all ((2048,2048) at 64
+    // rows, 16 stages: 11.6 us whole, 12.4 in two; (3000,2752) at 37, 22 stages: 13.6 -> 12.0 in three; (4096,4096), 32:
+    // 18.8 -> 14.4 in four; (4096,11008), 86: 42.8 -> 20.6 in four; (8192,8192), 64: 33.1 -> 23.6 in two)
+    if (pl.nb == 64) split = std::min(split, std::max(1, (kblocks - 7) / 5));
     if (g_tc_split > 0) split = std::min(g_tc_split, std::max(1, kblocks));
     if (v.tiles > 512) split = 1;  // the counter array holds 512 tiles x 4 row quarters
     pl.split = split;
@@ -199,6 +202,15 @@ static TcPlan plan_tc(const LayerView& v, int m) {
     const bool two_per_sm = pl.nb <= 128 && pl.tail_split <= 1 && (long long)v.tiles * pl.mtiles >= num_sms() * 6 / 5 &&
                             m <= 128;
     pl.dg = g_tc_dg > 0 ? std::min(g_tc_dg, 2) : (two_per_sm ? 1 : 2);
+    // More row tiles than SMs, two CTAs per SM: the tiles beyond a whole number per SM are cut along K, so that they do
+    // not cost a whole tile's time more on a few SMs ((57344,8192) at 128 rows, 448 tiles on 148 SMs: 143 -> 128.5 us;
+    // (28672,8192), 224 tiles: 75.9 -> 73.6)
+    const int units = v.tiles * pl.mtiles, slots = num_sms(), rest = units % slots;
+    if (two_per_sm && pl.split == 1 && g_tc_split == 0 && rest > 0 && stages_of(v) >= 32) {
+      pl.tail_split = rest * 4 <= slots ? 4 : rest * 3 <= slots ? 3 : 2;
+      pl.full_units = units - rest;
+      pl.tail_units = rest;
+    }
   }
   return pl;
 }
@@ -367,7 +379,7 @@ static int choose_kernel(const LayerView& v, int m, unsigned flags) {
   if (flags & QFB_FLAG_FORCE_SIMT) return 1;
   if (!tc_supported(v)) return 1;
   // K an odd multiple of 64: the CUDA-core kernel takes 8 rows a pass and reads the weights again for every 8 more
-  // ((3000,2752) at 37 rows: 79 us against 20)
+  // ((3000,2752) at 37 rows: 79 us against 12)
   if (v.k % 128 != 0) return m > kMaxSimtRows ? 2 : 1;
   if (flags & QFB_FLAG_FORCE_TENSOR) return 2;
   if (m >= g_tc_min_m) return 2;

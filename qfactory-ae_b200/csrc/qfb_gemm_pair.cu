@@ -133,37 +133,8 @@ struct PairTile {
 #pragma unroll
     for (int k = 0; k < 16; ++k) f[k] = __uint_as_float(v[k]);
   }
-  // 32 rows x 32 columns of the warp, rounded to fp16.  Three exchanges between lanes turn a row per lane into eight
-  // rows of four columns per lane: 4 stores of 16 bytes instead of 32 of 2.
   __device__ __forceinline__ void put(int c, const float (&f)[32]) const {
-    if (!vec) {
-#pragma unroll
-      for (int k = 0; k < 32; ++k)
-        if (c + k < cols && row_ok) y[(size_t)(c + k) * n_total + lane] = __float2half_rn(f[k]);
-      return;
-    }
-    uint32_t a[16], b[16];
-    const uint32_t sel = (lane & 1) ? 0x3276u : 0x5410u;
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {   // a[k]: column 2 k + bit 0 of the lane, rows (lane & ~1) ..+1
-      const uint32_t own = as_u32(__floats2half2_rn(f[2 * k], f[2 * k + 1]));
-      a[k] = prmt(own, __shfl_xor_sync(0xffffffffu, own, 1), sel);
-    }
-    const bool h2 = lane & 2, h4 = lane & 4;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {    // b[2 k ..]: column 4 k + bits 0, 1, rows (lane & ~3) ..+3
-      const uint32_t r = __shfl_xor_sync(0xffffffffu, h2 ? a[2 * k] : a[2 * k + 1], 2);
-      b[2 * k] = h2 ? r : a[2 * k];
-      b[2 * k + 1] = h2 ? a[2 * k + 1] : r;
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {    // column 8 k + bits 0, 1, 2, rows (lane & ~7) ..+7
-      const uint32_t r0 = __shfl_xor_sync(0xffffffffu, h4 ? b[4 * k] : b[4 * k + 2], 4);
-      const uint32_t r1 = __shfl_xor_sync(0xffffffffu, h4 ? b[4 * k + 1] : b[4 * k + 3], 4);
-      const uint4 v = h4 ? make_uint4(r0, r1, b[4 * k + 2], b[4 * k + 3]) : make_uint4(b[4 * k], b[4 * k + 1], r0, r1);
-      const int col = c + 8 * k + (lane & 7);
-      if (col < cols) *reinterpret_cast<uint4*>(y + (size_t)col * n_total + (lane & ~7)) = v;
-    }
+    put_rows<32>(y, n_total, c, cols, row_ok, vec, lane, f);
   }
   __device__ __forceinline__ void store(int c0, int step) const {
 #pragma unroll 1

@@ -76,6 +76,41 @@ struct TcCfg {
   static_assert(kDBase + (POST ? kRing * NB : kIssuers * NB) <= kTmemCols, "tensor memory over-subscribed");
 };
 
+// Sum of the split-K partials of one warp's 32 rows (lane = row) over all S splits, in split order,
+// rounded to fp16 into y, for the tiles with per-stage accumulators.  base0 -> partial of split 0, batch column 0, this
+// lane's row; `sstride` floats between splits, `cstride` between batch columns; ydst -> y[first batch row][this lane's
+// output feature], `ystride` halfs between batch rows; `cols` = valid batch columns.  8 columns of four splits are in
+// flight per round (a column at a time cost one round trip per column).
+template <int NB>
+__device__ __forceinline__ void splitk_reduce(const float* base0, size_t sstride, size_t cstride, int S, int cols,
+                                              bool row_ok, __half* ydst, size_t ystride) {
+  constexpr int CW = 8, SPB = 4;
+#pragma unroll 1
+  for (int c0 = 0; c0 < NB; c0 += CW) {
+    if (c0 >= cols) break;
+    float sum[CW];
+#pragma unroll
+    for (int j = 0; j < CW; ++j) sum[j] = 0.f;
+#pragma unroll 1
+    for (int sp = 0; sp < S; sp += SPB) {
+      float t[SPB][CW];
+#pragma unroll
+      for (int u = 0; u < SPB; ++u)
+#pragma unroll
+        for (int j = 0; j < CW; ++j)
+          t[u][j] = (sp + u < S && c0 + j < cols) ? __ldcg(base0 + (size_t)(sp + u) * sstride + (size_t)(c0 + j) * cstride) : 0.f;
+#pragma unroll
+      for (int u = 0; u < SPB; ++u)
+#pragma unroll
+        for (int j = 0; j < CW; ++j)
+          if (sp + u < S) sum[j] += t[u][j];
+    }
+#pragma unroll
+    for (int j = 0; j < CW; ++j)
+      if (c0 + j < cols && row_ok) ydst[(size_t)(c0 + j) * ystride] = __float2half_rn(sum[j]);
+  }
+}
+
 // FRAG = the layer is in the fragment layout (a build of its own: with both decoders behind a run-time branch in
 // the decode loop the compiler allots registers for the larger of the two)
 // ASYM = the layer has scales AND zero points (the common case; a build of its own for the same reason; used
@@ -93,6 +128,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
   __shared__ uint64_t bar_afull[R], bar_done[R], bar_dempty[R], bar_final;
   __shared__ uint32_t tmem_holder;
   __shared__ int abort_flag;
+  __shared__ unsigned tail_seen[4];   // per 32 rows: K ranges that have arrived / this one is the last
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Two grid shapes.  Uniform: grid (row tiles, batch tiles, K splits).  Tail-split (p.tail_split > 0,
@@ -316,43 +352,38 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
     const int row = q * 32 + lane;
     const int n = tile * kTileRows + row;
     const int m0 = mtile * NB;
-    // one 16-column chunk of results: fp16 output, or fp32 split-K partial
-    auto store_chunk = [&](int c, const float* v) {
+    if constexpr (POST) {
+      bool ok = true;
+      // one 16-column chunk of results: fp16 output, or fp32 split-K partial
+      auto store_chunk = [&](int c, const float* v) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int m = m0 + c + j;
-        if (m < p.m) {
-          if (S == 1) {
-            if (n < p.n) p.y[(size_t)m * p.n + n] = __float2half_rn(v[j]);
-          } else {
-            if (tail_unit >= 0) p.partial[(((size_t)split * p.tail_units + tail_unit) * NB + (c + j)) * kTileRows + row] = v[j];
-            else p.partial[((size_t)split * p.m + m) * p.npad + n] = v[j];
+        for (int j = 0; j < 16; ++j) {
+          const int m = m0 + c + j;
+          if (m < p.m) {
+            if (S == 1) {
+              if (n < p.n) p.y[(size_t)m * p.n + n] = __float2half_rn(v[j]);
+            } else {
+              p.partial[((size_t)split * p.m + m) * p.npad + n] = v[j];
+            }
           }
         }
-      }
-    };
-    bool ok = true;
-    // split-K: every epilogue warp publishes its 32 rows; per row quarter, the LAST warp to arrive
-    // over all splits sums that quarter's partials in split order (splitk_reduce)
-    auto finish_split = [&](uint32_t taddr_own, bool two) {
-      if (S <= 1) return;
-      __threadfence();
-      __syncwarp();
-      unsigned prev = 0;
-      unsigned* ctr = p.counters + (unit_ctr * 4 + q);
-      if (lane == 0) prev = atomicAdd(ctr, 1u);
-      prev = __shfl_sync(0xffffffffu, prev, 0);
-      if (prev != (unsigned)(S - 1)) return;
-      __threadfence();
-      const size_t sstride = tail_unit >= 0 ? (size_t)p.tail_units * NB * kTileRows : (size_t)p.m * p.npad;
-      const size_t cstride = tail_unit >= 0 ? (size_t)kTileRows : (size_t)p.npad;
-      const float* base0 = tail_unit >= 0 ? p.partial + (size_t)tail_unit * NB * kTileRows + row
-                                          : p.partial + (size_t)m0 * p.npad + n;
-      splitk_reduce<NB, POST>(base0, sstride, cstride, S, split, p.m - m0, n < p.n, p.y + (size_t)m0 * p.n + n, (size_t)p.n,
-                              taddr_own, two);
-      if (lane == 0) *ctr = 0u;
-    };
-    if (POST) {
+      };
+      // split-K: every epilogue warp publishes its 32 rows; per row quarter, the LAST warp to arrive
+      // over all splits sums that quarter's partials in split order (splitk_reduce)
+      auto finish_split = [&]() {
+        if (S <= 1) return;
+        __threadfence();
+        __syncwarp();
+        unsigned prev = 0;
+        unsigned* ctr = p.counters + (unit_ctr * 4 + q);
+        if (lane == 0) prev = atomicAdd(ctr, 1u);
+        prev = __shfl_sync(0xffffffffu, prev, 0);
+        if (prev != (unsigned)(S - 1)) return;
+        __threadfence();
+        splitk_reduce<NB>(p.partial + (size_t)m0 * p.npad + n, (size_t)p.m * p.npad, (size_t)p.npad, S, p.m - m0, n < p.n,
+                          p.y + (size_t)m0 * p.n + n, (size_t)p.n);
+        if (lane == 0) *ctr = 0u;
+      };
       float acc[NB];
 #pragma unroll
       for (int j = 0; j < NB; ++j) acc[j] = 0.f;
@@ -397,29 +428,116 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
         grid_dependency_wait();  // y and the workspace may still be in use by the preceding kernel
 #pragma unroll
         for (int c = 0; c < NB; c += 16) store_chunk(c, &acc[c]);
-        finish_split(0u, false);
+        finish_split();
       }
     } else {
-      ok = mbar_wait(smem_u32(&bar_final), 0, abortp, 500, wait_limit) && !*abortp;  // (an abandoned launch stores nothing)
-      if (ok) {
-        tc_fence_after();
-        grid_dependency_wait();
-        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + Cfg::kDBase;
-        const bool two = Cfg::kIssuers == 2 && nkb >= 2;  // the second accumulator holds something
-#pragma unroll 1
-        for (int c = 0; c < NB; c += 16) {
-          uint32_t v[16], v2[16];
-          tmem_ld_x16(taddr + c, v);
-          if (two) tmem_ld_x16(taddr + NB + c, v2);
-          tmem_wait_ld();
-          float f[16];
+      mbar_wait(smem_u32(&bar_final), 0, abortp, 500, wait_limit);   // (the results: all warps, below)
+    }
+  }
+
+  if constexpr (!POST) {
+    // ------------------------------ results, one accumulator over the K range: all warps ----
+    // (with the four epilogue warps alone a split of (2048,2048) at 64 rows cost 6 us: chains of dependent loads)
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (!*abortp) {   // (an abandoned launch stores nothing)
+      grid_dependency_wait();
+      const int q = warp & 3, m0 = mtile * NB, n0 = tile * kTileRows + q * 32, n = n0 + lane;
+      const int cols = min(NB, p.m - m0);
+      const int c0 = (warp >> 2) * 16;
+      constexpr int kStep = Cfg::kThreads / 128 * 16;
+      const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + Cfg::kDBase;
+      const bool two = Cfg::kIssuers == 2 && nkb >= 2;  // the second accumulator holds something
+      const bool vec = n0 + 32 <= p.n && p.n % 8 == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15u) == 0;
+      __half* y = p.y + (size_t)m0 * p.n + n0;
+      auto load16 = [&](int c, float (&f)[16]) {
+        uint32_t v[16], v2[16];
+        tmem_ld_x16(acc + c, v);
+        if (two) tmem_ld_x16(acc + NB + c, v2);
+        tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 16; ++j) f[j] = __uint_as_float(v[j]) + (two ? __uint_as_float(v2[j]) : 0.f);
-          store_chunk(c, f);
+        for (int k = 0; k < 16; ++k) f[k] = two ? __uint_as_float(v[k]) + __uint_as_float(v2[k]) : __uint_as_float(v[k]);
+      };
+      // partial sums: [range][unit][column][128] of the units that are cut, or [range][batch row][row]
+      const size_t sstride = tail_unit >= 0 ? (size_t)p.tail_units * NB * kTileRows : (size_t)p.m * p.npad;
+      const size_t cstride = tail_unit >= 0 ? (size_t)kTileRows : (size_t)p.npad;
+      float* part = tail_unit >= 0 ? p.partial + (size_t)tail_unit * NB * kTileRows + q * 32 + lane
+                                   : p.partial + (size_t)m0 * p.npad + n;
+      // the ranges in the order of K, the own one from tensor memory (the same bits) or, like the others, from memory
+      auto sum = [&](int own) {
+#pragma unroll 1
+        for (int c = c0; c < cols; c += kStep) {
+          float s[16];
+#pragma unroll
+          for (int k = 0; k < 16; ++k) s[k] = 0.f;
+#pragma unroll 1
+          for (int sp = 0; sp < S; ++sp) {
+            float f[16];
+            if (sp == own) {
+              load16(c, f);
+            } else {
+              const float* b = part + (size_t)sp * sstride + (size_t)c * cstride;
+#pragma unroll
+              for (int k = 0; k < 16; ++k) f[k] = c + k < cols ? __ldcg(b + (size_t)k * cstride) : 0.f;
+            }
+#pragma unroll
+            for (int k = 0; k < 16; ++k) s[k] += f[k];
+          }
+          put_rows<16>(y, p.n, c, cols, n < p.n, vec, lane, s);
         }
-        finish_split(taddr, two);
-        tc_fence_before();
+      };
+      if (S == 1) {
+#pragma unroll 1
+        for (int c = c0; c < cols; c += kStep) {
+          float f[16];
+          load16(c, f);
+          put_rows<16>(y, p.n, c, cols, n < p.n, vec, lane, f);
+        }
+      } else {
+        // the last range to arrive, per 32 rows, sums them all; one that finds the others there when it comes needs
+        // no partial sums of its own in memory
+        unsigned* ctr = p.counters + (unit_ctr * 4 + q);
+        if (warp < 4 && lane == 0) {
+          unsigned seen;
+          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(ctr) : "memory");
+          tail_seen[q] = seen;
+        }
+        __syncthreads();
+        const bool there = tail_seen[q] == (unsigned)(S - 1);
+        if (there) {
+          sum(split);
+        } else {
+#pragma unroll 1
+          for (int c = c0; c < cols; c += kStep) {
+            float f[16];
+            load16(c, f);
+            float* b = part + (size_t)split * sstride + (size_t)c * cstride;
+#pragma unroll
+            for (int k = 0; k < 16; ++k)
+              if (c + k < cols) __stcg(b + (size_t)k * cstride, f[k]);
+          }
+          __threadfence();
+        }
+        __syncthreads();
+        if (warp < 4 && lane == 0) {
+          if (there) {
+            *ctr = 0u;
+            tail_seen[q] = 0u;
+          } else {
+            __threadfence();
+            tail_seen[q] = atomicAdd(ctr, 1u) == (unsigned)(S - 1) ? 1u : 0u;
+            __threadfence();
+          }
+        }
+        __syncthreads();
+        if (tail_seen[q]) {
+          __threadfence();
+          sum(-1);
+          if (warp < 4 && lane == 0) *ctr = 0u;
+        }
       }
+      tc_fence_before();
     }
   }
 

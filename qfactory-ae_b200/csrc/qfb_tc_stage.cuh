@@ -203,60 +203,39 @@ template <> struct StageDecode<3> {
   }
 };
 
-// Sum of the split-K partials of one warp's 32 rows (lane = row) over all S splits, in split order,
-// rounded to fp16 into y.  base0 -> partial of split 0, batch column 0, this lane's row; `sstride`
-// floats between splits, `cstride` between batch columns; ydst -> y[first batch row][this lane's
-// output feature], `ystride` halfs between batch rows; `cols` = valid batch columns.
-// Loads in flight per round: 32 batch columns of one split where one accumulator spans K (this
-// warp's own sums, the same bits it published, are re-read from tensor memory at taddr_own instead,
-// plus the second issuer's accumulator when `two`); 8 columns of four splits for the narrow
-// per-stage-accumulator tiles, which have many splits.  (A column at a time cost one round trip per
-// column: the reduce of a wide tile then took longer than its MMAs.  Measured against 16 columns of
-// two splits and against a non-inlined function: this form is 2-7 % faster on every batch size.)
-template <int NB, bool POST>
-__device__ __forceinline__ void splitk_reduce(const float* base0, size_t sstride, size_t cstride, int S, int split, int cols,
-                                           bool row_ok, __half* ydst, size_t ystride, uint32_t taddr_own, bool two) {
-  constexpr int CW = POST ? 8 : 32, SPB = POST ? 4 : 1;
-#pragma unroll 1
-  for (int c0 = 0; c0 < NB; c0 += CW) {
-    if (c0 >= cols) break;
-    float sum[CW];
+// 32 rows (lane = row) x W columns of a warp, rounded to fp16 into y[column][row] (y: column 0, first row of the warp).
+// With `vec` (whole 8-row runs inside the layer, every y row 16-byte aligned) three exchanges between lanes turn a row
+// per lane into eight rows of W / 8 columns per lane: W / 8 stores of 16 bytes instead of W of 2.
+template <int W>
+__device__ __forceinline__ void put_rows(__half* y, int n_total, int c, int cols, bool row_ok, bool vec, int lane,
+                                         const float (&f)[W]) {
+  if (!vec) {
 #pragma unroll
-    for (int j = 0; j < CW; ++j) sum[j] = 0.f;
-#pragma unroll 1
-    for (int sp = 0; sp < S; sp += SPB) {
-      float t[SPB][CW];
+    for (int k = 0; k < W; ++k)
+      if (c + k < cols && row_ok) y[(size_t)(c + k) * n_total + lane] = __float2half_rn(f[k]);
+    return;
+  }
+  uint32_t a[W / 2], b[W / 2];
+  const uint32_t sel = (lane & 1) ? 0x3276u : 0x5410u;
 #pragma unroll
-      for (int u = 0; u < SPB; ++u) {
-        if (!POST && sp + u == split) continue;   // filled below, without a load
+  for (int k = 0; k < W / 2; ++k) {   // a[k]: column 2 k + bit 0 of the lane, rows (lane & ~1) ..+1
+    const uint32_t own = as_u32(__floats2half2_rn(f[2 * k], f[2 * k + 1]));
+    a[k] = prmt(own, __shfl_xor_sync(0xffffffffu, own, 1), sel);
+  }
+  const bool h2 = lane & 2, h4 = lane & 4;
 #pragma unroll
-        for (int j = 0; j < CW; ++j)
-          t[u][j] = (sp + u < S && c0 + j < cols) ? __ldcg(base0 + (size_t)(sp + u) * sstride + (size_t)(c0 + j) * cstride) : 0.f;
-      }
-      if (!POST) {
+  for (int k = 0; k < W / 4; ++k) {    // b[2 k ..]: column 4 k + bits 0, 1, rows (lane & ~3) ..+3
+    const uint32_t r = __shfl_xor_sync(0xffffffffu, h2 ? a[2 * k] : a[2 * k + 1], 2);
+    b[2 * k] = h2 ? r : a[2 * k];
+    b[2 * k + 1] = h2 ? a[2 * k + 1] : r;
+  }
 #pragma unroll
-        for (int u = 0; u < SPB; ++u)
-          if (sp + u == split) {
-#pragma unroll
-            for (int c = 0; c < CW; c += 16) {
-              uint32_t v[16], v2[16];
-              tmem_ld_x16(taddr_own + c0 + c, v);
-              if (two) tmem_ld_x16(taddr_own + NB + c0 + c, v2);
-              tmem_wait_ld();
-#pragma unroll
-              for (int j = 0; j < 16; ++j) t[u][c + j] = __uint_as_float(v[j]) + (two ? __uint_as_float(v2[j]) : 0.f);
-            }
-          }
-      }
-#pragma unroll
-      for (int u = 0; u < SPB; ++u)
-#pragma unroll
-        for (int j = 0; j < CW; ++j)
-          if (sp + u < S) sum[j] += t[u][j];
-    }
-#pragma unroll
-    for (int j = 0; j < CW; ++j)
-      if (c0 + j < cols && row_ok) ydst[(size_t)(c0 + j) * ystride] = __float2half_rn(sum[j]);
+  for (int k = 0; k < W / 8; ++k) {    // column 8 k + bits 0, 1, 2, rows (lane & ~7) ..+7
+    const uint32_t r0 = __shfl_xor_sync(0xffffffffu, h4 ? b[4 * k] : b[4 * k + 2], 4);
+    const uint32_t r1 = __shfl_xor_sync(0xffffffffu, h4 ? b[4 * k + 1] : b[4 * k + 3], 4);
+    const uint4 v = h4 ? make_uint4(r0, r1, b[4 * k + 2], b[4 * k + 3]) : make_uint4(b[4 * k], b[4 * k + 1], r0, r1);
+    const int col = c + 8 * k + (lane & 7);
+    if (col < cols) *reinterpret_cast<uint4*>(y + (size_t)col * n_total + (lane & ~7)) = v;
   }
 }
 
