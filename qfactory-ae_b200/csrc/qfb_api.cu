@@ -346,10 +346,10 @@ static int run_tc(const LayerView& v, const __half* x, int m, __half* y, void* w
     if (workspace && ws_bytes >= need) {
       p.counters = reinterpret_cast<unsigned*>(static_cast<char*>(workspace) + kHeaderBytes);
       p.partial = reinterpret_cast<float*>(static_cast<char*>(workspace) + off);
-    } else if (v.k % 128 == 0) {
+    } else if (v.k % 128 == 0 && (pl.post || p.kblocks >= 160)) {
       return QFB_ERR_WORKSPACE;
     } else {
-      split = 1;   // (these sizes also run with the smaller workspace of the CUDA-core kernel)
+      split = 1;   // (an optimisation here: without room for the partial sums every range runs whole)
     }
   }
   dim3 grid(v.tiles, pl.mtiles, split);

@@ -69,3 +69,19 @@ def test_without_room_for_partial_sums_units_run_whole():
     # fp32 sums in another order, both rounded to fp16
     bound = 2.0 ** -9 * y.float().abs() + k / 16 * 2.0 ** -22 * y.float().abs().max()
     assert bool(((y.float() - y2.float()).abs() <= bound).all())
+
+
+def test_split_tiles_of_33_to_64_rows_without_a_workspace():
+    m, n, k = 40, 1000, 4096
+    g = torch.Generator(device="cuda").manual_seed(6)
+    codes = torch.randint(0, 16, (k, n), generator=g, dtype=torch.int32, device="cuda")
+    s = (torch.rand(k // 128, n, generator=g, device="cuda") * 0.018 + 0.002).half()
+    layer = QLinear.init(m, k, n, 4, codes, 128, s, None)
+    x = torch.randn(m, k, generator=g, device="cuda").half()
+    y = layer(x)
+    assert _native.last_launch()["grid_y"] > 1
+    layer._ws_bytes = 4096   # (such calls ran whole, and without a workspace, before their K was split)
+    y2 = layer(x)
+    assert _native.last_launch()["grid_y"] == 1
+    bound = 2.0 ** -9 * y.float().abs() + k / 16 * 2.0 ** -22 * y.float().abs().max()
+    assert bool(((y.float() - y2.float()).abs() <= bound).all())
