@@ -268,7 +268,7 @@ qgemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   if (warp == 0) {
     // ------------------------------ weight producer ---------------------------
     if (lane == 0) {
-      if constexpr (kSwizzledStage<BITS, FRAG>) prefetch_tensormap(&tmap_w);
+      if constexpr (kSwizzledStage<BITS, FRAG, false>) prefetch_tensormap(&tmap_w);
       const int hpg = p.halfstages_per_group;
       const uint32_t ng = hpg == 1 ? 2u : 1u;
       const uint32_t zb = has_z ? ng * 128u : 0u, sb = has_s ? ng * 256u : 0u;
@@ -290,7 +290,7 @@ qgemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
           const uint32_t zn = half && hpg == 1 ? zb / 2 : zb, sn = half && hpg == 1 ? sb / 2 : sb;
           mbar_arrive_expect_tx(bar, wb + zn + sn + ((p.stall_test && at == s_begin + j.nkb && i == 0) ? 16u : 0u));
           const uint32_t dst = sbase + w_off + s * Cfg::kWBytes;
-          if constexpr (kSwizzledStage<BITS, FRAG>) {
+          if constexpr (kSwizzledStage<BITS, FRAG, false>) {
             const int r0 = (tile * 2 * p.kblocks + j.kb0 + i) * (16 * BITS);
             tma_tensor_2d_g2s(dst, &tmap_w, 0, r0, bar);
             tma_tensor_2d_g2s(dst + Cfg::kWBytes / 2, &tmap_w, 0, r0 + p.kblocks * (16 * BITS), bar);
@@ -389,7 +389,7 @@ qgemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       if (!mbar_wait(smem_u32(&bar_wfull[s]), (uint32_t)(i / NS) & 1u, abortp, kSleepDecode, wait_limit)) break;
       const uint32_t z = has_z ? (uint32_t)gbase[z_off + s * Cfg::kZSlot + qrow] : p.zconst;
       __half2 d[32];
-      if constexpr (FRAG) StageDecodeFragment<BITS>::run(gbase + w_off + s * Cfg::kWBytes, row, h, z, d);
+      if constexpr (FRAG) StageDecodeFragment<BITS, kSwizzledStage<BITS, FRAG, false>>::run(gbase + w_off + s * Cfg::kWBytes, row, h, z, d);
       else StageDecode<BITS>::run(gbase + w_off + s * Cfg::kWBytes, row, h, z, d);
       uint32_t rr[32];
       if (has_s) {

@@ -203,7 +203,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
     // ------------------------------ weight producer ---------------------------
     // (depends on the preceding kernel only where TcParams::early is not set: the wait above)
     if (lane == 0) {
-      if constexpr (kSwizzledStage<BITS, FRAG>) prefetch_tensormap(&tmap_w);
+      if constexpr (kSwizzledStage<BITS, FRAG, POST>) prefetch_tensormap(&tmap_w);
       const uint8_t* wsrc = reinterpret_cast<const uint8_t*>(p.qw) + (size_t)tile * p.k * (16 * BITS) + (size_t)kb0 * Cfg::kWBytes;
       int s = 0;
       uint32_t ph = 1;  // first pass over the ring: parity 1 of a fresh barrier passes at once
@@ -221,7 +221,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
         const uint32_t zn = half && hpg == 1 ? zb / 2 : zb, sn = half && hpg == 1 ? sb / 2 : sb;
         // zeros / scales of the groups this stage touches: one group, or two when the group is 64
         mbar_arrive_expect_tx(bar, wb + zn + sn + ((p.stall_test && i == 0) ? 16u : 0u));
-        if constexpr (kSwizzledStage<BITS, FRAG>) {
+        if constexpr (kSwizzledStage<BITS, FRAG, POST>) {
           // the stage is two runs: 8 k-steps (2 * BITS rows of 64 bytes each) of the upper and of the lower 64 rows
           const int r0 = (tile * 2 * p.kblocks + kb0 + i) * (16 * BITS);
           tma_tensor_2d_g2s(sbase + w_off + s * Cfg::kWBytes, &tmap_w, 0, r0, bar);
@@ -310,7 +310,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
       if (!mbar_wait(smem_u32(&bar_wfull[s]), phs, abortp, kSleepDecode, wait_limit)) break;
       const uint32_t z = has_z ? (uint32_t)gbase[z_off + s * Cfg::kZSlot + qrow] : p.zconst;
       __half2 d[32];
-      if constexpr (FRAG) StageDecodeFragment<BITS>::run(gbase + w_off + s * Cfg::kWBytes, row, h, z, d);
+      if constexpr (FRAG) StageDecodeFragment<BITS, kSwizzledStage<BITS, FRAG, POST>>::run(gbase + w_off + s * Cfg::kWBytes, row, h, z, d);
       else StageDecode<BITS>::run(gbase + w_off + s * Cfg::kWBytes, row, h, z, d);
       uint32_t rr[32];
       if (!POST && has_s) {

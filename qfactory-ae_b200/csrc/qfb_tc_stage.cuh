@@ -20,8 +20,9 @@ constexpr unsigned kSleepScale = 100, kSleepProducer = 100, kSleepMma = 20, kSle
 // reads, 512 shared-memory cycles a stage beside the MMAs' and the copies' own ((28672,8192) at 64 / 1024 rows 67.5
 // -> 62 and 580 -> 491 us, (8192,28672) at 128 rows 85 -> 75 us).  Not for 2 bits, whose words are 32 bytes apart
 // (2-way, and 32-byte rows would double the copy's requests), nor for 3, whose planes are read without conflicts
-// inside a row block.
-template <int BITS, bool FRAG> constexpr bool kSwizzledStage = FRAG && (BITS == 4 || BITS == 8);
+// inside a row block; nor with per-stage accumulators (up to 32 rows), which wait for the copies and not for the decode:
+// copies of 64-byte rows are slower than two bulk copies ((8192,8192) 8-bit at 24 rows 27.7 us against 25.4).
+template <int BITS, bool FRAG, bool POST> constexpr bool kSwizzledStage = FRAG && !POST && (BITS == 4 || BITS == 8);
 
 // ---- decode of the 64 codes thread (row, h) owns in a 128-k stage -> 32 fp16 pairs ------
 template <int BITS> struct StageDecode;
@@ -46,10 +47,10 @@ template <> struct StageDecode<4> {
 // Fragment layouts: stage = [2 halves of 64 rows][8 k-steps of 128 * BITS bytes] (qfb_common.cuh).
 // Row wt*64 + rb*16 + hh*8 + g owns, in the word frag_word_of(rb, hh) of lane g*4+t, the codes of
 // k 4t..4t+3 of a step: two exact fp16 pairs in k order per word.
-// For 4 and 8 bits the 64 bytes of a g (the words of t 0..3, 16 bytes each) arrive 64-byte-swizzled
-// (kSwizzledStage): the chunk of t sits at t ^ (g >> 1).
-template <int BITS> struct StageDecodeFragment;
-template <> struct StageDecodeFragment<4> {
+// SWZ (kSwizzledStage): the 64 bytes of a g (the words of t 0..3, 16 bytes each) arrived 64-byte-swizzled: the chunk
+// of t sits at t ^ (g >> 1).
+template <int BITS, bool SWZ> struct StageDecodeFragment;
+template <bool SWZ> struct StageDecodeFragment<4, SWZ> {
   // nibbles 0,4,2,6 (hh = 0) or 1,5,3,7 (hh = 1): two LOP3 with the row's mask / magic
   __device__ static __forceinline__ void run(const uint8_t* w, int row, int h, uint32_t z, __half2 (&d)[32]) {
     const Codec<4>::ZM zm = Codec<4>::zmagic(z);
@@ -61,13 +62,13 @@ template <> struct StageDecodeFragment<4> {
     for (int ks = 0; ks < 4; ++ks)
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
-        const uint32_t word = *reinterpret_cast<const uint32_t*>(base + ks * 512 + ((t ^ (g >> 1)) << 4));
+        const uint32_t word = *reinterpret_cast<const uint32_t*>(base + ks * 512 + ((SWZ ? t ^ (g >> 1) : t) << 4));
         d[ks * 8 + t * 2] = __hsub2(as_h2(lop3_and_or(word, mask, magic)), zs);
         d[ks * 8 + t * 2 + 1] = __hsub2(as_h2(lop3_and_or(word >> 8, mask, magic)), zs);
       }
   }
 };
-template <> struct StageDecodeFragment<8> {
+template <bool SWZ> struct StageDecodeFragment<8, SWZ> {
   // one word = the row's four bytes of k 4t..4t+3
   __device__ static __forceinline__ void run(const uint8_t* w, int row, int h, uint32_t z, __half2 (&d)[32]) {
     const Codec<8>::ZM zm = Codec<8>::zmagic(z);
@@ -77,13 +78,13 @@ template <> struct StageDecodeFragment<8> {
     for (int ks = 0; ks < 4; ++ks)
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
-        const uint32_t word = *reinterpret_cast<const uint32_t*>(base + ks * 1024 + ((t ^ (g >> 1)) << 4));
+        const uint32_t word = *reinterpret_cast<const uint32_t*>(base + ks * 1024 + ((SWZ ? t ^ (g >> 1) : t) << 4));
         d[ks * 8 + t * 2] = __hsub2(as_h2(prmt(word, 0x64646464u, 0x4140u)), as_h2(zm.m));
         d[ks * 8 + t * 2 + 1] = __hsub2(as_h2(prmt(word, 0x64646464u, 0x4342u)), as_h2(zm.m));
       }
   }
 };
-template <> struct StageDecodeFragment<2> {
+template <bool SWZ> struct StageDecodeFragment<2, SWZ> {
   // one word = two row blocks; the row's fields sit at bit o = 4 (rb & 1) + 2 hh of each byte pair
   __device__ static __forceinline__ void run(const uint8_t* w, int row, int h, uint32_t z, __half2 (&d)[32]) {
     const Codec<2>::ZM zm = Codec<2>::zmagic(z);
@@ -103,7 +104,7 @@ template <> struct StageDecodeFragment<2> {
       }
   }
 };
-template <> struct StageDecodeFragment<3> {
+template <bool SWZ> struct StageDecodeFragment<3, SWZ> {
   // word j of lane g*4+t sits in plane j (128 bytes) of the k-step (384 bytes).  Row blocks 0..2: word rb, the
   // row's fields at bit offset 0 (rows g) or 3 (rows g + 8) for k 4t, 4t+1 and 9 bits higher for k 4t+2, 4t+3.
   // Row block 3: offset 6 of words 0 / 1 (rows g) and of word 2 (rows g + 8, k 4t, 4t+1); rows g + 8,
