@@ -20,8 +20,8 @@ constexpr unsigned kSleepScale = 100, kSleepProducer = 100, kSleepMma = 20, kSle
 // reads, 512 shared-memory cycles a stage beside the MMAs' and the copies' own ((28672,8192) at 64 / 1024 rows 67.5
 // -> 62 and 580 -> 491 us, (8192,28672) at 128 rows 85 -> 75 us).  Not for 2 bits, whose words are 32 bytes apart
 // (2-way, and 32-byte rows would double the copy's requests), nor for 3, whose planes are read without conflicts
-// inside a row block; nor with per-stage accumulators (up to 32 rows), which wait for the copies and not for the decode:
-// copies of 64-byte rows are slower than two bulk copies ((8192,8192) 8-bit at 24 rows 27.7 us against 25.4).
+// inside a row block; nor with per-stage accumulators (up to 32 rows), where it changes nothing ((8192,8192)
+// 8-bit at 24 rows 27.7 us with it, 27.6 without).
 template <int BITS, bool FRAG, bool POST> constexpr bool kSwizzledStage = FRAG && !POST && (BITS == 4 || BITS == 8);
 
 // ---- decode of the 64 codes thread (row, h) owns in a 128-k stage -> 32 fp16 pairs ------
