@@ -7,15 +7,19 @@
 //
 // Every entry serves the plain case (dense fp16 CUDA tensors on the current device, contiguous) and returns
 // NotImplemented for anything else; the Python code that called it then takes its general path, which also raises
-// the errors.  A status other than QFB_OK comes back as an int.  The C ABI is reached through function addresses that
-// the binding passes in, so this module does not link the library.
+// the errors.  A status other than QFB_OK comes back as an int.  What torch throws (no memory for an output, a tensor
+// without storage) becomes the Python exception torch's own bindings raise: no C++ exception reaches the interpreter's
+// frames.  The C ABI is reached through function addresses that the binding passes in, so this module does not link
+// the library.
 #include <Python.h>
 #include <structmember.h>
 
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/object_ptr.h>
 
 #include "../../include/qfactory_b200.h"
 
@@ -49,6 +53,12 @@ struct LayerCall {
 };
 
 inline PyObject* general() { Py_RETURN_NOTIMPLEMENTED; }
+
+// the GIL given up for the time of a launch, and taken back on any way out
+struct WithoutGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~WithoutGil() { PyEval_RestoreThread(state); }
+};
 
 // the plain tensor behind `o`, or null where a subclass or another object needs the general path
 inline const at::Tensor* plain(PyObject* o) {
@@ -91,9 +101,10 @@ PyObject* run_linear(LayerCall* L, PyObject* xo, PyObject* outo, bool fused) {
   void *yp = y.mutable_data_ptr(), *st = stream_of(L->device);
   const linear_fn fn = fused ? abi.linear_silu_mul : abi.linear;
   int status;
-  Py_BEGIN_ALLOW_THREADS  // a launch waits where the stream's queue is full
-  status = fn(&L->desc, xp, (int)rows, yp, L->ws, (size_t)L->ws_bytes, L->flags, st);
-  Py_END_ALLOW_THREADS
+  {
+    WithoutGil released;  // a launch waits where the stream's queue is full
+    status = fn(&L->desc, xp, (int)rows, yp, L->ws, (size_t)L->ws_bytes, L->flags, st);
+  }
   if (outo && outo != Py_None && status == 0) {
     Py_INCREF(outo);
     return outo;
@@ -127,12 +138,16 @@ void layer_dealloc(PyObject* self) {
 }
 
 PyObject* layer_forward(PyObject* self, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
   if (na < 1 || na > 2) return general();
   return run_linear(reinterpret_cast<LayerCall*>(self), a[0], na > 1 ? a[1] : nullptr, false);
+  END_HANDLE_TH_ERRORS
 }
 PyObject* layer_forward_silu_mul(PyObject* self, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
   if (na < 1 || na > 2) return general();
   return run_linear(reinterpret_cast<LayerCall*>(self), a[0], na > 1 ? a[1] : nullptr, true);
+  END_HANDLE_TH_ERRORS
 }
 
 PyMethodDef layer_methods[] = {
@@ -157,6 +172,7 @@ inline bool empty_container(PyObject* o) {
 }
 
 PyObject* call_layer(PyObject*, PyObject* const* a, Py_ssize_t na, PyObject* kwnames) {
+  HANDLE_TH_ERRORS
   // layer(x), layer(x, out) or layer(x, out=...)
   PyObject* self = na > 0 ? a[0] : nullptr;
   const Py_ssize_t nkw = kwnames ? PyTuple_GET_SIZE(kwnames) : 0;
@@ -170,35 +186,29 @@ PyObject* call_layer(PyObject*, PyObject* const* a, Py_ssize_t na, PyObject* kwn
     PyObject** dictp = ok ? _PyObject_GetDictPtr(self) : nullptr;
     PyObject* dict = nullptr;
     if (ok && dictp) dict = *dictp;
-    PyObject* owned = nullptr;
-    if (ok && !dict) dict = owned = PyObject_GenericGetDict(self, nullptr);
+    THPObjectPtr owned, native;
+    if (ok && !dict) {
+      owned = PyObject_GenericGetDict(self, nullptr);
+      dict = owned.get();
+    }
     if (ok && dict) {
       for (Py_ssize_t i = 0; ok && i < PyTuple_GET_SIZE(hook_keys); ++i)
         ok = empty_container(PyDict_GetItem(dict, PyTuple_GET_ITEM(hook_keys, i)));
       ok = ok && PyDict_GetItem(dict, key_forward) == nullptr;
-      PyObject* native = ok ? PyDict_GetItem(dict, key_native) : nullptr;
-      if (native && Py_TYPE(native) == &LayerType) {
-        Py_INCREF(native);
-        PyObject* y = run_linear(reinterpret_cast<LayerCall*>(native), a[1], na + nkw > 2 ? a[2] : nullptr, false);
-        Py_DECREF(native);
-        if (y && THPVariable_Check(y)) {
-          Py_XDECREF(owned);
-          return y;
-        }
-        if (!y) {
-          Py_XDECREF(owned);
-          return nullptr;
-        }
+      native = ok ? Py_XNewRef(PyDict_GetItem(dict, key_native)) : nullptr;
+      if (native && Py_TYPE(native.get()) == &LayerType) {
+        PyObject* y = run_linear(reinterpret_cast<LayerCall*>(native.get()), a[1], na + nkw > 2 ? a[2] : nullptr, false);
+        if (!y || THPVariable_Check(y)) return y;
         Py_DECREF(y);  // NotImplemented or a status: the Python path repeats the call and raises what is wrong
       }
     }
-    Py_XDECREF(owned);
   }
   if (!module_call) {
     PyErr_SetString(PyExc_RuntimeError, "_qfb_torch.bind has not been called");
     return nullptr;
   }
   return PyObject_Vectorcall(module_call, a, (size_t)na, kwnames);
+  END_HANDLE_TH_ERRORS
 }
 
 // ---- element-wise neighbours ---------------------------------------------------------------------------------
@@ -223,6 +233,7 @@ inline PyObject* give(int st, PyObject* o, at::Tensor& y) {
 
 // rmsnorm(x, residual | None, weight, eps, out | None)
 PyObject* py_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
   if (na != 5) return general();
   const at::Tensor *x = plain(a[0]), *w = plain(a[2]);
   const bool add = a[1] != Py_None;
@@ -238,15 +249,18 @@ PyObject* py_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
   void *xp = x->data_ptr(), *yp = y.mutable_data_ptr(), *st = stream_of(dev);
   const void *wp = w->data_ptr(), *rp = add ? r->data_ptr() : nullptr;
   int status;
-  Py_BEGIN_ALLOW_THREADS
-  status = add ? abi.add_rmsnorm(xp, rp, wp, yp, (int)rows, (int)d, (float)eps, st)
-               : abi.rmsnorm(xp, wp, yp, (int)rows, (int)d, (float)eps, st);
-  Py_END_ALLOW_THREADS
+  {
+    WithoutGil released;
+    status = add ? abi.add_rmsnorm(xp, rp, wp, yp, (int)rows, (int)d, (float)eps, st)
+                 : abi.rmsnorm(xp, wp, yp, (int)rows, (int)d, (float)eps, st);
+  }
   return give(status, a[4], y);
+  END_HANDLE_TH_ERRORS
 }
 
 // silu_mul(gate_up, out | None)
 PyObject* py_silu_mul(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
   if (na != 2) return general();
   const at::Tensor* x = plain(a[0]);
   if (!x || !x->is_cuda() || x->dim() < 1) return general();
@@ -261,14 +275,17 @@ PyObject* py_silu_mul(PyObject*, PyObject* const* a, Py_ssize_t na) {
   const void* xp = x->data_ptr();
   void *yp = y.mutable_data_ptr(), *st = stream_of(dev);
   int status;
-  Py_BEGIN_ALLOW_THREADS
-  status = abi.silu_mul(xp, yp, (int)rows, (int)half, st);
-  Py_END_ALLOW_THREADS
+  {
+    WithoutGil released;
+    status = abi.silu_mul(xp, yp, (int)rows, (int)half, st);
+  }
   return give(status, a[1], y);
+  END_HANDLE_TH_ERRORS
 }
 
 // decode_attention_rope(qkv, cos, sin, pos, k_cache, v_cache, q_heads, kv_heads, out | None)
 PyObject* py_attention_rope(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
   if (na != 9) return general();
   const at::Tensor* t[6];
   for (int i = 0; i < 6; ++i)
@@ -290,10 +307,12 @@ PyObject* py_attention_rope(PyObject*, PyObject* const* a, Py_ssize_t na) {
   const void *qp = qkv.data_ptr(), *cp = cosv.data_ptr(), *sp = sinv.data_ptr(), *pp = pos.data_ptr();
   const int max_len = (int)kc.size(2);
   int status;
-  Py_BEGIN_ALLOW_THREADS
-  status = abi.attention_rope(qp, cp, sp, pp, kp, vp, yp, (int)B, (int)hq, (int)hkv, (int)hd, max_len, st);
-  Py_END_ALLOW_THREADS
+  {
+    WithoutGil released;
+    status = abi.attention_rope(qp, cp, sp, pp, kp, vp, yp, (int)B, (int)hq, (int)hkv, (int)hd, max_len, st);
+  }
   return give(status, a[8], y);
+  END_HANDLE_TH_ERRORS
 }
 
 // bind(addresses: dict, module_call, served_types: tuple, global_hooks: tuple, hook_keys: tuple)
