@@ -242,7 +242,12 @@ PyObject* py_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
   const int dev = x->get_device();
   if (!dense_half(*x, dev) || w->scalar_type() != at::kHalf || !w->is_cuda() || !on_current(dev)) return general();
   if (add && (!dense_half(*r, dev) || r->sizes() != x->sizes())) return general();
+  if (!PyFloat_Check(a[3]) && !PyLong_Check(a[3])) return general();  // (what is no number is for ctypes to refuse)
   const double eps = PyFloat_AsDouble(a[3]);
+  if (eps == -1.0 && PyErr_Occurred()) {
+    PyErr_Clear();
+    return general();
+  }
   const int64_t d = x->sizes().back(), rows = d ? x->numel() / d : 0;
   at::Tensor y;
   if (rows > INT32_MAX || d > INT32_MAX || !out_tensor(a[4], x->sizes(), dev, &y)) return general();
@@ -292,7 +297,12 @@ PyObject* py_attention_rope(PyObject*, PyObject* const* a, Py_ssize_t na) {
     if (!(t[i] = plain(a[i])) || !t[i]->is_cuda() || !t[i]->is_contiguous()) return general();
   const at::Tensor &qkv = *t[0], &cosv = *t[1], &sinv = *t[2], &pos = *t[3], &kc = *t[4], &vc = *t[5];
   const int dev = qkv.get_device();
+  if (!PyLong_Check(a[6]) || !PyLong_Check(a[7])) return general();
   const long hq = PyLong_AsLong(a[6]), hkv = PyLong_AsLong(a[7]);
+  if ((hq == -1 || hkv == -1) && PyErr_Occurred()) {
+    PyErr_Clear();
+    return general();
+  }
   if (!dense_half(qkv, dev) || !on_current(dev) || qkv.dim() != 4 || qkv.size(1) != 1 || qkv.size(2) != hq + 2 * hkv)
     return general();
   if (pos.scalar_type() != at::kLong || pos.numel() != 1 || cosv.scalar_type() != at::kHalf || sinv.scalar_type() != at::kHalf)
