@@ -14,11 +14,15 @@
 #include <Python.h>
 #include <structmember.h>
 
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/PyInterpreter.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/utils/object_ptr.h>
 
 #include "../../include/qfactory_b200.h"
@@ -67,8 +71,21 @@ inline const at::Tensor* plain(PyObject* o) {
 inline bool dense_half(const at::Tensor& t, int device) {
   return t.is_cuda() && t.scalar_type() == at::kHalf && t.get_device() == device && t.is_contiguous();
 }
+// Something looks at torch's operations (a tracer, functorch, a dispatch or function mode): the Python path, whose
+// operations it sees.  A default device is a function mode too, but concerns only factory calls that name no device.
+PyObject* device_context_type = nullptr;
+inline bool observed() {
+  if (torch::jit::tracer::isTracing()) return true;
+  const c10::DispatchKeySet included = c10::impl::tls_local_dispatch_key_set().included_;
+  if (!(included - c10::default_included_set).empty()) return true;
+  for (int64_t i = at::impl::PythonTorchFunctionTLS::stack_len() - 1; i >= 0; --i) {
+    PyObject* mode = at::impl::PythonTorchFunctionTLS::get_stack_at(i)->ptr(getPyInterpreter());
+    if (reinterpret_cast<PyObject*>(Py_TYPE(mode)) != device_context_type) return true;
+  }
+  return false;
+}
 // launches go to the current device: the plain case is the one where it is the tensors' own
-inline bool on_current(int device) { return c10::cuda::current_device() == device; }
+inline bool ordinary(int device) { return c10::cuda::current_device() == device && !observed(); }
 inline void* stream_of(int device) { return c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream(); }
 
 inline at::Tensor empty_half(c10::IntArrayRef sizes, int device) {
@@ -78,7 +95,7 @@ inline at::Tensor empty_half(c10::IntArrayRef sizes, int device) {
 // One linear: x [..., width] -> y [..., n].  `fused` = x is [gate | up] and the layer's input is silu(gate) * up.
 PyObject* run_linear(LayerCall* L, PyObject* xo, PyObject* outo, bool fused) {
   const at::Tensor* x = plain(xo);
-  if (!x || !dense_half(*x, L->device) || !on_current(L->device)) return general();
+  if (!x || !dense_half(*x, L->device) || !ordinary(L->device)) return general();
   const int64_t width = (int64_t)L->desc.k * (fused ? 2 : 1), n = L->desc.n;
   const auto sizes = x->sizes();
   if (sizes.empty() || sizes.back() != width) return general();
@@ -162,52 +179,85 @@ PyTypeObject LayerType = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
 // ---- `layer(x)` without torch.nn.Module.__call__ -------------------------------------------------------------
 // nn.Module's call walks several Python frames to find that a layer has no hooks (1-2 us).  This function is the
-// layers' `__call__`: where neither the module nor torch as a whole has a hook, a compiled call, or a replaced
-// `forward`, it runs the layer; anything else goes to nn.Module's own.
-PyObject *module_call = nullptr, *served_types = nullptr, *global_hooks = nullptr;
-PyObject *key_native = nullptr, *key_forward = nullptr, *hook_keys = nullptr;
+// layers' `__call__`: where the call that a layer inherits, its `_call_impl` and its `forward` are the ones they were
+// when the classes were made, and neither the module nor torch as a whole has a hook or a compiled call, it runs the
+// layer; anything else goes to the inherited call as it is at that moment, so that a replaced nn.Module.__call__ (as
+// torch.fx's tracer does) or `forward` is seen.
+PyObject *layer_call_method = nullptr;   // this function, as it stands in the classes
+PyObject *served = nullptr;              // ((class, its forward, its _call_impl), ...)
+PyObject *plain_call = nullptr;          // nn.Module's own __call__
+PyObject *global_hooks = nullptr, *hook_keys = nullptr;
+PyObject *key_native = nullptr, *key_forward = nullptr, *key_call = nullptr, *key_call_impl = nullptr;
 
 inline bool empty_container(PyObject* o) {
   return o == nullptr || o == Py_None || (PyDict_Check(o) && PyDict_Size(o) == 0);
 }
 
+// the `__call__` behind this module's own in the order of the type's bases (borrowed)
+PyObject* inherited_call(PyTypeObject* type) {
+  bool own = false;
+  PyObject* mro = type->tp_mro;
+  for (Py_ssize_t i = 0; mro && i < PyTuple_GET_SIZE(mro); ++i) {
+    PyObject* dict = reinterpret_cast<PyTypeObject*>(PyTuple_GET_ITEM(mro, i))->tp_dict;
+    PyObject* call = dict ? PyDict_GetItem(dict, key_call) : nullptr;
+    if (own && call && call != layer_call_method) return call;
+    own = own || call == layer_call_method;
+  }
+  return nullptr;
+}
+
+// the call object of a layer that nobody has hooked, wrapped or replaced a part of; null otherwise
+THPObjectPtr unhooked(PyObject* self, PyObject* inherited) {
+  if (inherited != plain_call) return THPObjectPtr();
+  bool ok = false;
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(served) && !ok; ++i) {
+    PyObject* entry = PyTuple_GET_ITEM(served, i);
+    ok = reinterpret_cast<PyObject*>(Py_TYPE(self)) == PyTuple_GET_ITEM(entry, 0) &&
+         _PyType_Lookup(Py_TYPE(self), key_forward) == PyTuple_GET_ITEM(entry, 1) &&
+         _PyType_Lookup(Py_TYPE(self), key_call_impl) == PyTuple_GET_ITEM(entry, 2);
+  }
+  for (Py_ssize_t i = 0; ok && i < PyTuple_GET_SIZE(global_hooks); ++i) ok = empty_container(PyTuple_GET_ITEM(global_hooks, i));
+  if (!ok) return THPObjectPtr();
+  PyObject** dictp = _PyObject_GetDictPtr(self);
+  THPObjectPtr dict(dictp && *dictp ? Py_NewRef(*dictp) : PyObject_GenericGetDict(self, nullptr));
+  if (!dict) {
+    PyErr_Clear();
+    return THPObjectPtr();
+  }
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(hook_keys); ++i)
+    if (!empty_container(PyDict_GetItem(dict.get(), PyTuple_GET_ITEM(hook_keys, i)))) return THPObjectPtr();
+  PyObject* native = PyDict_GetItem(dict.get(), key_native);
+  return native && Py_TYPE(native) == &LayerType ? THPObjectPtr(Py_NewRef(native)) : THPObjectPtr();
+}
+
 PyObject* call_layer(PyObject*, PyObject* const* a, Py_ssize_t na, PyObject* kwnames) {
   HANDLE_TH_ERRORS
-  // layer(x), layer(x, out) or layer(x, out=...)
-  PyObject* self = na > 0 ? a[0] : nullptr;
-  const Py_ssize_t nkw = kwnames ? PyTuple_GET_SIZE(kwnames) : 0;
-  const bool form = (na == 2 && nkw == 0) || (na == 3 && nkw == 0) ||
-                    (na == 2 && nkw == 1 && PyUnicode_CompareWithASCIIString(PyTuple_GET_ITEM(kwnames, 0), "out") == 0);
-  if (form && module_call) {
-    bool ok = false;
-    for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(served_types) && !ok; ++i)
-      ok = reinterpret_cast<PyObject*>(Py_TYPE(self)) == PyTuple_GET_ITEM(served_types, i);
-    for (Py_ssize_t i = 0; ok && i < PyTuple_GET_SIZE(global_hooks); ++i) ok = empty_container(PyTuple_GET_ITEM(global_hooks, i));
-    PyObject** dictp = ok ? _PyObject_GetDictPtr(self) : nullptr;
-    PyObject* dict = nullptr;
-    if (ok && dictp) dict = *dictp;
-    THPObjectPtr owned, native;
-    if (ok && !dict) {
-      owned = PyObject_GenericGetDict(self, nullptr);
-      dict = owned.get();
-    }
-    if (ok && dict) {
-      for (Py_ssize_t i = 0; ok && i < PyTuple_GET_SIZE(hook_keys); ++i)
-        ok = empty_container(PyDict_GetItem(dict, PyTuple_GET_ITEM(hook_keys, i)));
-      ok = ok && PyDict_GetItem(dict, key_forward) == nullptr;
-      native = ok ? Py_XNewRef(PyDict_GetItem(dict, key_native)) : nullptr;
-      if (native && Py_TYPE(native.get()) == &LayerType) {
-        PyObject* y = run_linear(reinterpret_cast<LayerCall*>(native.get()), a[1], na + nkw > 2 ? a[2] : nullptr, false);
-        if (!y || THPVariable_Check(y)) return y;
-        Py_DECREF(y);  // NotImplemented or a status: the Python path repeats the call and raises what is wrong
-      }
-    }
-  }
-  if (!module_call) {
-    PyErr_SetString(PyExc_RuntimeError, "_qfb_torch.bind has not been called");
+  if (!served || na < 1) {
+    PyErr_SetString(PyExc_RuntimeError, "_qfb_torch: no layer, or bind has not been called");
     return nullptr;
   }
-  return PyObject_Vectorcall(module_call, a, (size_t)na, kwnames);
+  PyObject *self = a[0], *inherited = inherited_call(Py_TYPE(self));
+  if (!inherited) {
+    PyErr_Format(PyExc_TypeError, "'%.200s' object is not a layer", Py_TYPE(self)->tp_name);
+    return nullptr;
+  }
+  // layer(x), layer(x, out) or layer(x, out=...)
+  const Py_ssize_t nkw = kwnames ? PyTuple_GET_SIZE(kwnames) : 0;
+  if ((na == 2 && nkw == 0) || (na == 3 && nkw == 0) ||
+      (na == 2 && nkw == 1 && PyUnicode_CompareWithASCIIString(PyTuple_GET_ITEM(kwnames, 0), "out") == 0)) {
+    THPObjectPtr native = unhooked(self, inherited);
+    if (native) {
+      PyObject* y = run_linear(reinterpret_cast<LayerCall*>(native.get()), a[1], na + nkw > 2 ? a[2] : nullptr, false);
+      if (!y || THPVariable_Check(y)) return y;
+      Py_DECREF(y);  // NotImplemented or a status: the Python path repeats the call and raises what is wrong
+    }
+  }
+  THPObjectPtr call(Py_NewRef(inherited));
+  if (PyType_HasFeature(Py_TYPE(call.get()), Py_TPFLAGS_METHOD_DESCRIPTOR))
+    return PyObject_Vectorcall(call.get(), a, (size_t)na, kwnames);
+  const descrgetfunc get = Py_TYPE(call.get())->tp_descr_get;
+  THPObjectPtr bound(get ? get(call.get(), self, reinterpret_cast<PyObject*>(Py_TYPE(self))) : Py_NewRef(call.get()));
+  return bound ? PyObject_Vectorcall(bound.get(), a + 1, (size_t)(na - 1), kwnames) : nullptr;
   END_HANDLE_TH_ERRORS
 }
 
@@ -240,7 +290,7 @@ PyObject* py_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
   const at::Tensor* r = add ? plain(a[1]) : nullptr;
   if (!x || !w || (add && !r) || !x->is_cuda() || x->dim() < 1) return general();
   const int dev = x->get_device();
-  if (!dense_half(*x, dev) || w->scalar_type() != at::kHalf || !w->is_cuda() || !on_current(dev)) return general();
+  if (!dense_half(*x, dev) || w->scalar_type() != at::kHalf || !w->is_cuda() || !ordinary(dev)) return general();
   if (add && (!dense_half(*r, dev) || r->sizes() != x->sizes())) return general();
   if (!PyFloat_Check(a[3]) && !PyLong_Check(a[3])) return general();  // (what is no number is for ctypes to refuse)
   const double eps = PyFloat_AsDouble(a[3]);
@@ -271,7 +321,7 @@ PyObject* py_silu_mul(PyObject*, PyObject* const* a, Py_ssize_t na) {
   if (!x || !x->is_cuda() || x->dim() < 1) return general();
   const int dev = x->get_device();
   const int64_t half = x->sizes().back() / 2;
-  if (!dense_half(*x, dev) || !on_current(dev) || half < 1) return general();
+  if (!dense_half(*x, dev) || !ordinary(dev) || half < 1) return general();
   const int64_t rows = x->numel() / (2 * half);
   c10::SmallVector<int64_t, 6> shape(x->sizes().begin(), x->sizes().end());
   shape.back() = half;
@@ -303,7 +353,7 @@ PyObject* py_attention_rope(PyObject*, PyObject* const* a, Py_ssize_t na) {
     PyErr_Clear();
     return general();
   }
-  if (!dense_half(qkv, dev) || !on_current(dev) || qkv.dim() != 4 || qkv.size(1) != 1 || qkv.size(2) != hq + 2 * hkv)
+  if (!dense_half(qkv, dev) || !ordinary(dev) || qkv.dim() != 4 || qkv.size(1) != 1 || qkv.size(2) != hq + 2 * hkv)
     return general();
   if (pos.scalar_type() != at::kLong || pos.numel() != 1 || cosv.scalar_type() != at::kHalf || sinv.scalar_type() != at::kHalf)
     return general();
@@ -325,12 +375,18 @@ PyObject* py_attention_rope(PyObject*, PyObject* const* a, Py_ssize_t na) {
   END_HANDLE_TH_ERRORS
 }
 
-// bind(addresses: dict, module_call, served_types: tuple, global_hooks: tuple, hook_keys: tuple)
+// bind(addresses: dict, nn.Module's __call__, ((class, forward, _call_impl), ...), global_hooks: tuple, hook_keys: tuple,
+//      the function mode of a default device)
 PyObject* py_bind(PyObject*, PyObject* args) {
-  PyObject *addr, *mc, *types, *globals, *keys;
-  if (!PyArg_ParseTuple(args, "O!OO!O!O!", &PyDict_Type, &addr, &mc, &PyTuple_Type, &types, &PyTuple_Type, &globals, &PyTuple_Type,
-                        &keys))
+  PyObject *addr, *mc, *types, *globals, *keys, *devctx;
+  if (!PyArg_ParseTuple(args, "O!OO!O!O!O", &PyDict_Type, &addr, &mc, &PyTuple_Type, &types, &PyTuple_Type, &globals,
+                        &PyTuple_Type, &keys, &devctx))
     return nullptr;
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(types); ++i)
+    if (!PyTuple_Check(PyTuple_GET_ITEM(types, i)) || PyTuple_GET_SIZE(PyTuple_GET_ITEM(types, i)) != 3) {
+      PyErr_SetString(PyExc_ValueError, "a served class comes with its forward and its _call_impl");
+      return nullptr;
+    }
   auto at_name = [&](const char* n) -> void* {
     PyObject* v = PyDict_GetItemString(addr, n);
     return v ? PyLong_AsVoidPtr(v) : nullptr;
@@ -345,11 +401,12 @@ PyObject* py_bind(PyObject*, PyObject* args) {
     if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "an entry point is missing");
     return nullptr;
   }
-  for (PyObject* o : {mc, types, globals, keys}) Py_INCREF(o);
-  Py_XSETREF(module_call, mc);
-  Py_XSETREF(served_types, types);
+  for (PyObject* o : {mc, types, globals, keys, devctx}) Py_INCREF(o);
+  Py_XSETREF(plain_call, mc);
+  Py_XSETREF(served, types);
   Py_XSETREF(global_hooks, globals);
   Py_XSETREF(hook_keys, keys);
+  Py_XSETREF(device_context_type, devctx);
   Py_RETURN_NONE;
 }
 
@@ -378,11 +435,14 @@ PyMODINIT_FUNC PyInit__qfb_torch(void) {
   if (PyType_Ready(&LayerType) < 0) return nullptr;
   key_native = PyUnicode_InternFromString("_native_call");
   key_forward = PyUnicode_InternFromString("forward");
+  key_call = PyUnicode_InternFromString("__call__");
+  key_call_impl = PyUnicode_InternFromString("_call_impl");
   PyObject* m = PyModule_Create(&module_def);
-  if (!m || !key_native || !key_forward) return nullptr;
+  if (!m || !key_native || !key_forward || !key_call || !key_call_impl) return nullptr;
   PyObject* call = PyObject_GetAttrString(m, "call_layer");
   PyObject* method = call ? PyInstanceMethod_New(call) : nullptr;  // binds to the instance as a Python function would
   Py_XDECREF(call);
+  layer_call_method = Py_XNewRef(method);
   Py_INCREF(&LayerType);
   if (!method || PyModule_AddObject(m, "layer_call_method", method) < 0 ||
       PyModule_AddObject(m, "LayerCall", reinterpret_cast<PyObject*>(&LayerType)) < 0) {

@@ -195,14 +195,20 @@ def lib() -> ctypes.CDLL:
 
 
 _torch_module = None
-_layer_types = ()
+_served = ()
+_plain_call = None
 
 
 def serve_types(*types) -> None:
     """Layer classes whose `__call__` becomes the native one when the module below is loaded (exactly these
-    classes: a subclass may bring a `forward` of its own)."""
-    global _layer_types
-    _layer_types = types
+    classes: a subclass may bring a `forward` of its own).  What they inherit is noted now, when the classes are
+    made: a call that finds something else in its place goes the ordinary way."""
+    global _served, _plain_call
+    import torch
+
+    # (nn.Module's call under its second name, which nothing that wraps calls for a while replaces)
+    _plain_call = torch.nn.Module._wrapped_call_impl
+    _served = tuple((t, t.forward, t._call_impl) for t in types)
 
 
 def torch_module():
@@ -214,6 +220,7 @@ def torch_module():
         import importlib.util
 
         import torch.nn.modules.module as tm
+        from torch.utils._device import DeviceContext
 
         if not os.path.exists(TORCH_MODULE_PATH):
             raise NativeError(f"native module {TORCH_MODULE_PATH} not found: build it with "
@@ -229,10 +236,14 @@ def torch_module():
         # and the module's
         hooks = tuple(getattr(tm, n) for n in ("_global_backward_pre_hooks", "_global_backward_hooks", "_global_forward_hooks",
                                                "_global_forward_pre_hooks"))
-        keys = ("_backward_hooks", "_backward_pre_hooks", "_forward_hooks", "_forward_pre_hooks", "_compiled_call_impl")
-        m.bind({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in names}, tm.Module.__call__, _layer_types, hooks, keys)
-        for t in _layer_types:
-            t.__call__ = m.layer_call_method
+        # ... and what a module may carry in the place of its class's own
+        keys = ("_backward_hooks", "_backward_pre_hooks", "_forward_hooks", "_forward_pre_hooks", "_compiled_call_impl",
+                "forward", "_call_impl")
+        m.bind({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in names}, _plain_call, _served, hooks, keys,
+               DeviceContext)
+        for t, _, _ in _served:
+            if "__call__" not in t.__dict__:
+                t.__call__ = m.layer_call_method
         _torch_module = m
     return _torch_module
 

@@ -43,3 +43,58 @@ def test_what_torch_throws_is_a_python_exception():
     lines = r.stdout.split("\n")
     assert r.returncode == 0 and "alive" in lines, (r.returncode, r.stdout[-500:], r.stderr[-800:])
     assert sum(line.startswith("raised") for line in lines) == 6, r.stdout
+
+
+def _layers():
+    from qfactory import QLinear
+
+    _native.torch_module()   # (its `__call__` is in the classes from here on)
+    return [QLinear.empty(1, 256, 128, 4, 128, False, device="cpu"), QLinear.empty(1, 256, 128, 4, -1, True, device="cpu")]
+
+
+def test_a_wrapped_module_call_sees_the_layers():
+    import torch
+
+    for layer in _layers():
+        net = torch.nn.Sequential(layer, torch.nn.ReLU())
+
+        class Tracer(torch.fx.Tracer):
+            def is_leaf_module(self, m, name):
+                return m is layer or super().is_leaf_module(m, name)
+
+        graph = Tracer().trace(net)
+        assert [n.op for n in graph.nodes] == ["placeholder", "call_module", "call_module", "output"]
+
+
+def test_calls_go_where_python_would_send_them():
+    import torch
+
+    seen = []
+
+    class Mixin(torch.nn.Module):
+        def __call__(self, *a, **kw):
+            seen.append("mixin")
+            return super().__call__(*a, **kw)
+
+    for layer in _layers():
+        cls = type(layer)
+
+        class Sub(cls, Mixin):
+            def __call__(self, *a, **kw):
+                seen.append("sub")
+                return super().__call__(*a, **kw)
+
+            def forward(self, x, out=None):
+                return ("forward", x, out)
+
+        sub = Sub.__new__(Sub)
+        sub.__dict__.update(layer.__dict__)
+        seen.clear()
+        assert sub(1, out=2) == ("forward", 1, 2) and seen == ["sub", "mixin"]
+        assert sub(1, 3) == ("forward", 1, 3) and sub(x=4) == ("forward", 4, None)
+        with pytest.raises(TypeError):
+            sub()
+        with pytest.raises(_native.NativeError):   # no CPU path
+            layer(torch.zeros(1, 256, dtype=torch.float16))
+        with pytest.raises(TypeError):
+            cls.__call__(object(), 1)
