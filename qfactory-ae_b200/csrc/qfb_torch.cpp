@@ -281,26 +281,24 @@ inline PyObject* give(int st, PyObject* o, at::Tensor& y) {
   return THPVariable_Wrap(std::move(y));
 }
 
-// rmsnorm(x, residual | None, weight, eps, out | None)
-PyObject* py_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
-  HANDLE_TH_ERRORS
-  if (na != 5) return general();
-  const at::Tensor *x = plain(a[0]), *w = plain(a[2]);
-  const bool add = a[1] != Py_None;
-  const at::Tensor* r = add ? plain(a[1]) : nullptr;
+// `ro`: the residual, or null for the norm alone
+PyObject* run_rmsnorm(PyObject* xo, PyObject* ro, PyObject* wo, PyObject* epso, PyObject* outo) {
+  const at::Tensor *x = plain(xo), *w = plain(wo);
+  const bool add = ro != nullptr;
+  const at::Tensor* r = add ? plain(ro) : nullptr;
   if (!x || !w || (add && !r) || !x->is_cuda() || x->dim() < 1) return general();
   const int dev = x->get_device();
   if (!dense_half(*x, dev) || w->scalar_type() != at::kHalf || !w->is_cuda() || !ordinary(dev)) return general();
   if (add && (!dense_half(*r, dev) || r->sizes() != x->sizes())) return general();
-  if (!PyFloat_Check(a[3]) && !PyLong_Check(a[3])) return general();  // (what is no number is for ctypes to refuse)
-  const double eps = PyFloat_AsDouble(a[3]);
+  if (!PyFloat_Check(epso) && !PyLong_Check(epso)) return general();  // (what is no number is for ctypes to refuse)
+  const double eps = PyFloat_AsDouble(epso);
   if (eps == -1.0 && PyErr_Occurred()) {
     PyErr_Clear();
     return general();
   }
   const int64_t d = x->sizes().back(), rows = d ? x->numel() / d : 0;
   at::Tensor y;
-  if (rows > INT32_MAX || d > INT32_MAX || !out_tensor(a[4], x->sizes(), dev, &y)) return general();
+  if (rows > INT32_MAX || d > INT32_MAX || !out_tensor(outo, x->sizes(), dev, &y)) return general();
   void *xp = x->data_ptr(), *yp = y.mutable_data_ptr(), *st = stream_of(dev);
   const void *wp = w->data_ptr(), *rp = add ? r->data_ptr() : nullptr;
   int status;
@@ -309,7 +307,20 @@ PyObject* py_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
     status = add ? abi.add_rmsnorm(xp, rp, wp, yp, (int)rows, (int)d, (float)eps, st)
                  : abi.rmsnorm(xp, wp, yp, (int)rows, (int)d, (float)eps, st);
   }
-  return give(status, a[4], y);
+  return give(status, outo, y);
+}
+
+// rmsnorm(x, weight, eps, out | None)
+PyObject* py_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  return na == 4 ? run_rmsnorm(a[0], nullptr, a[1], a[2], a[3]) : general();
+  END_HANDLE_TH_ERRORS
+}
+
+// add_rmsnorm(x, residual, weight, eps, out | None)
+PyObject* py_add_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  return na == 5 ? run_rmsnorm(a[0], a[1], a[2], a[3], a[4]) : general();
   END_HANDLE_TH_ERRORS
 }
 
@@ -413,7 +424,8 @@ PyObject* py_bind(PyObject*, PyObject* args) {
 PyMethodDef methods[] = {
     {"bind", py_bind, METH_VARARGS, "addresses of the C ABI and the state of torch.nn.Module's call"},
     {"call_layer", reinterpret_cast<PyCFunction>(call_layer), METH_FASTCALL | METH_KEYWORDS, "__call__ of the layers"},
-    {"rmsnorm", reinterpret_cast<PyCFunction>(py_rmsnorm), METH_FASTCALL, "rmsnorm(x, residual, weight, eps, out)"},
+    {"rmsnorm", reinterpret_cast<PyCFunction>(py_rmsnorm), METH_FASTCALL, "rmsnorm(x, weight, eps, out)"},
+    {"add_rmsnorm", reinterpret_cast<PyCFunction>(py_add_rmsnorm), METH_FASTCALL, "add_rmsnorm(x, residual, weight, eps, out)"},
     {"silu_mul", reinterpret_cast<PyCFunction>(py_silu_mul), METH_FASTCALL, "silu_mul(gate_up, out)"},
     {"decode_attention_rope", reinterpret_cast<PyCFunction>(py_attention_rope), METH_FASTCALL,
      "decode_attention_rope(qkv, cos, sin, pos, k_cache, v_cache, q_heads, kv_heads, out)"},

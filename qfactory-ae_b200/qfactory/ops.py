@@ -17,7 +17,7 @@ def _stream(t):
 
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5, out: torch.Tensor | None = None) -> torch.Tensor:
     """fp16(x * rsqrt(mean(x^2, -1) + eps)) * weight over the last dimension."""
-    y = _native.torch_module().rmsnorm(x, None, weight, eps, out)
+    y = _native.torch_module().rmsnorm(x, weight, eps, out)
     if isinstance(y, torch.Tensor):
         return y
     assert x.is_cuda and x.dtype == torch.float16 and x.is_contiguous() and weight.dtype == torch.float16
@@ -32,7 +32,7 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5, out: torch
 def add_rmsnorm(x: torch.Tensor, residual: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5,
                 out: torch.Tensor | None = None) -> torch.Tensor:
     """x += residual (in place, fp16), then the RMS norm of the sum: returns the normed tensor."""
-    y = _native.torch_module().rmsnorm(x, residual, weight, eps, out)
+    y = _native.torch_module().add_rmsnorm(x, residual, weight, eps, out)
     if isinstance(y, torch.Tensor):
         return y
     assert x.is_cuda and x.dtype == torch.float16 and x.is_contiguous()

@@ -28,6 +28,15 @@ def test_an_eps_that_is_no_number_is_refused(eps):
     assert torch.equal(ops.rmsnorm(x, w, 1), ops.rmsnorm(x, w, 1.0))
 
 
+def test_the_sum_with_no_residual_is_refused():
+    x, w = torch.randn(2, 256, device="cuda").half(), torch.ones(256, device="cuda").half()
+    before = x.clone()
+    for none in (None, x[:1], x.float()):
+        with pytest.raises((AttributeError, AssertionError)):
+            ops.add_rmsnorm(x, none, w)
+    assert torch.equal(x, before)
+
+
 def test_head_counts_that_are_no_numbers_are_refused():
     qkv = torch.zeros(1, 1, 3, 128, dtype=torch.float16, device="cuda")
     cos = sin = torch.zeros(8, 64, dtype=torch.float16, device="cuda")
