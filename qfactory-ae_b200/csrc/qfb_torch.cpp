@@ -105,6 +105,7 @@ PyObject* run_linear(LayerCall* L, PyObject* xo, PyObject* outo, bool fused) {
   if (outo && outo != Py_None) {
     const at::Tensor* o = plain(outo);
     if (!o || !dense_half(*o, L->device) || o->numel() != rows * n || sizes.size() != 2) return general();
+    if (fused && (o->dim() != 2 || o->size(1) != n)) return general();  // (comes back in the shape of the rows)
     y = *o;
   } else if (sizes.size() == 2) {
     const int64_t shape[2] = {rows, n};

@@ -165,6 +165,20 @@ def test_outputs_ranks_strides_and_streams():
     assert torch.equal(layer(x), want)
 
 
+@pytest.mark.parametrize("m", [1, 6])
+def test_the_fused_activation_gives_the_shape_of_the_rows(m):
+    layer, _ = _layer(m=m)
+    gu = torch.randn(m, 1024, device="cuda").half()
+    want = layer.forward_silu_mul(gu)
+    assert want.shape == (m, 256) and torch.equal(want, layer(ops.silu_mul(gu)))
+    for shape in ((m, 256), (m * 256,), (1, m, 256), (m * 2, 128)):
+        out = torch.empty(shape, dtype=torch.float16, device="cuda")
+        y = layer.forward_silu_mul(gu, out)
+        assert y.shape == (m, 256) and y.data_ptr() == out.data_ptr() and torch.equal(y, want)
+    y = layer.forward_silu_mul(gu.view(m, 1, 1024), torch.empty_like(want))
+    assert y.shape == (m, 1, 256) and torch.equal(y.view(m, 256), want)
+
+
 def test_flags_and_workspace_changed_after_the_first_call():
     from qfactory import _native
 
