@@ -1044,7 +1044,7 @@ int qfb_quantize_pack(const void* weight, int n, int k, int bits, int group_size
   if (st != QFB_OK) return st;
   if (group_size == -1) return QFB_ERR_BAD_SHAPE;
   if (!weight || !zeros_out || !range_flags) return QFB_ERR_NULL_POINTER;
-  if (reinterpret_cast<uintptr_t>(weight) & 3u) return QFB_ERR_MISALIGNED;
+  if (reinterpret_cast<uintptr_t>(weight) & 1u) return QFB_ERR_MISALIGNED;
   p.weight = static_cast<const __half*>(weight);
   p.qz = static_cast<uint8_t*>(zeros_out);
   return check_cuda(launch_quantize_pack(p, static_cast<cudaStream_t>(stream)));

@@ -385,7 +385,8 @@ __global__ void __launch_bounds__(kPackThreads, 4) quantize_pack_kernel(const Pa
   __shared__ __half2 ext[2][4][64];   // largest and smallest value per quarter and pair of rows
   const int tile = blockIdx.x, n0 = tile * kTileRows, kbeg = blockIdx.y * run, kend = min(kbeg + run, p.k);
   const int c = threadIdx.x & 63, h = threadIdx.x >> 6, n = n0 + 2 * c;
-  const bool pair = n + 1 < p.n && (p.n & 1) == 0;   // both rows exist and every row of the source is aligned to pairs
+  // both rows exist and every row of the source is aligned to pairs (the source itself may begin at any fp16 value)
+  const bool pair = n + 1 < p.n && (p.n & 1) == 0 && (reinterpret_cast<uintptr_t>(p.weight) & 3u) == 0;
   constexpr int kLevels = (1 << BITS) - 1;
   const int gs = p.group_size;
   unsigned bad = 0;

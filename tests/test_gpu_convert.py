@@ -36,6 +36,16 @@ def test_float_weight(bits, group, K, N, layout):
     _same(QLinear.from_float(w.cuda(), bits, group, layout=layout), QLinear.init(1, K, N, bits, q, group, s, z, layout=layout))
 
 
+@pytest.mark.parametrize("bits,group,K,N", [(4, 64, 192, 200), (8, 128, 256, 131)])
+def test_float_weight_at_an_odd_place_of_a_buffer(bits, group, K, N):
+    w = torch.randn(K, N, generator=torch.Generator().manual_seed(N)).half()
+    flat = torch.empty(K * N + 1, dtype=torch.float16, device="cuda")
+    view = flat[1:].view(K, N)
+    view.copy_(w)
+    assert view.is_contiguous() and view.data_ptr() % 4 == 2
+    _same(QLinear.from_float(view, bits, group), QLinear.from_float(w, bits, group))
+
+
 @pytest.mark.parametrize("sym", [False, True])
 @pytest.mark.parametrize("bits,group,K,N", [c for c in CASES if c[0] != 3 and c[3] % 16 == 0 or c[3] == 1000])
 def test_gptq_words(bits, group, K, N, sym):
