@@ -181,8 +181,9 @@ __device__ __forceinline__ uint8_t effective_zero(int z, int bits) { return (uin
 template <int BITS, int SRC, bool FRAG>
 __global__ void __launch_bounds__(kPackThreads) pack_kernel(const PackParams p) {
   __shared__ __align__(16) uint32_t s[kTileRows * kPackRow];
-  // (row tiles fastest: concurrent CTAs read whole rows of the source)
-  const int tile = blockIdx.x, n0 = tile * kTileRows, k0 = blockIdx.y * kPackK, klen = min(kPackK, p.k - k0);
+  // (row tiles fastest: concurrent CTAs read whole rows of the source; one grid dimension, which has room for any K)
+  const int tile = blockIdx.x % p.tiles, n0 = tile * kTileRows;
+  const int k0 = (int)(blockIdx.x / p.tiles) * kPackK, klen = min(kPackK, p.k - k0);
   unsigned bad = stage_codes<BITS, SRC>(p, s, n0, k0, klen);
   // scales and zeros of the groups that begin in this block (at most two)
   if (p.qs) {
@@ -215,7 +216,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(const PackParams p) 
 
 template <int BITS>
 static cudaError_t launch_pack_bits(const PackParams& p, cudaStream_t st) {
-  const dim3 grid(p.tiles, (p.k + kPackK - 1) / kPackK);
+  const unsigned grid = (unsigned)p.tiles * ((p.k + kPackK - 1) / kPackK);
   const bool frag = p.layout == QFB_LAYOUT_FRAGMENT;
   if (p.gptq_codes) {
     if constexpr (BITS != 3) {
@@ -383,7 +384,8 @@ template <int BITS, bool FRAG>
 __global__ void __launch_bounds__(kPackThreads, 4) quantize_pack_kernel(const PackParams p, int run) {
   __shared__ __align__(16) uint32_t s[kTileRows * kPackRow];
   __shared__ __half2 ext[2][4][64];   // largest and smallest value per quarter and pair of rows
-  const int tile = blockIdx.x, n0 = tile * kTileRows, kbeg = blockIdx.y * run, kend = min(kbeg + run, p.k);
+  const int tile = blockIdx.x % p.tiles, n0 = tile * kTileRows;
+  const int kbeg = (int)(blockIdx.x / p.tiles) * run, kend = min(kbeg + run, p.k);
   const int c = threadIdx.x & 63, h = threadIdx.x >> 6, n = n0 + 2 * c;
   // both rows exist and every row of the source is aligned to pairs (the source itself may begin at any fp16 value)
   const bool pair = n + 1 < p.n && (p.n & 1) == 0 && (reinterpret_cast<uintptr_t>(p.weight) & 3u) == 0;
@@ -488,7 +490,7 @@ __global__ void __launch_bounds__(kPackThreads, 4) quantize_pack_kernel(const Pa
 template <int BITS>
 static cudaError_t launch_quantize_pack_bits(const PackParams& p, cudaStream_t st) {
   const int run = p.group_size == 64 ? 128 : p.group_size;
-  const dim3 grid(p.tiles, (p.k + run - 1) / run);
+  const unsigned grid = (unsigned)p.tiles * ((p.k + run - 1) / run);
   if (p.layout == QFB_LAYOUT_FRAGMENT) quantize_pack_kernel<BITS, true><<<grid, kPackThreads, 0, st>>>(p, run);
   else quantize_pack_kernel<BITS, false><<<grid, kPackThreads, 0, st>>>(p, run);
   return cudaGetLastError();

@@ -71,3 +71,22 @@ def test_values_out_of_range_are_reported():
             convert_params(args, (q.cuda(), s.cuda(), z2.cuda()))
     with pytest.raises(AssertionError, match="zero"):   # a group far below zero has a zero point no code can hold
         QLinear.from_float(torch.full((K, N), -3.0).half().cuda() + torch.rand(K, N).half().cuda(), 4, group)
+
+
+def test_more_blocks_along_k_than_a_grid_has_in_its_second_dimension():
+    # 65536 blocks of 128: the last of them must hold what a layer made of the last rows alone holds
+    K, N, tail = 65536 * 128, 8, 1024
+    g = torch.Generator(device="cuda").manual_seed(9)
+    w = torch.randn(K, N, generator=g, dtype=torch.float16, device="cuda")
+    q = torch.randint(0, 16, (K, N), generator=g, dtype=torch.int32, device="cuda")
+    s = torch.rand(K // 128, N, generator=g, device="cuda").half()
+    words = torch.randint(-2 ** 31, 2 ** 31, (K // 8, N), generator=g, dtype=torch.int64, device="cuda").to(torch.int32)
+    for make in (lambda a: QLinear.from_float(w[-a:], 4, 128, layout="tile"),
+                 lambda a: QLinear.init(1, a, N, 4, q[-a:], 128, s[-(a // 128):], None, layout="tile"),
+                 lambda a: gptq.layer_from_gptq(words[-(a // 8):], None, s[-(a // 128):], 4, 128, sym=True)):
+        whole, last = make(K), make(tail)
+        if whole.packed_layout == last.packed_layout == 0:   # tile layout: the units of the one row tile follow each other
+            assert torch.equal(whole.w.view(-1)[-last.w.numel():], last.w.view(-1))
+        else:                                                # fragment layout: a run for each half of the tile
+            assert torch.equal(whole.w.view(2, -1)[:, -(last.w.numel() // 2):], last.w.view(2, -1))
+        assert torch.equal(whole.s.view(-1)[-last.s.numel():], last.s.view(-1))
