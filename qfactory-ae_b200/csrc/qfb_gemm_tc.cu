@@ -389,7 +389,8 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
       for (int j = 0; j < NB; ++j) acc[j] = 0.f;
       const size_t sz_row = (size_t)tile * p.groups * kTileRows +
                             (FRAG ? frag_pos_of_row(row) : row);
-      const int stages_per_group = p.halfstages_per_group >> 1;  // POST needs groups of whole stages
+      // (POST needs groups of whole stages, but for a group-less layer of K = 64: half a stage)
+      const int stages_per_group = max(1, p.halfstages_per_group >> 1);
       int r = 0;
       uint32_t phr = 0;
       // scales are fetched two stages ahead of their use

@@ -30,7 +30,7 @@ def _check(y, x, w):
 
 
 @pytest.mark.parametrize("m,n,k,bits,group,sym", [
-    (9, 200, 192, 4, 64, False), (16, 128, 64, 8, 64, True), (17, 1000, 1088, 2, -1, True), (32, 256, 704, 4, -1, True),
+    (9, 200, 192, 4, 64, False), (16, 128, 64, 8, 64, True), (16, 200, 64, 4, -1, True), (32, 128, 64, 2, -1, True), (17, 1000, 1088, 2, -1, True), (32, 256, 704, 4, -1, True),
     (37, 3000, 2752, 4, 64, False), (64, 384, 4160, 8, 64, False), (65, 300, 1344, 2, 64, True), (128, 19200, 320, 4, 64, False),
     (200, 8192, 11072, 4, 64, False), (300, 9472, 2752, 8, -1, True), (600, 640, 2112, 4, 64, True)])
 def test_half_filled_last_stage(m, n, k, bits, group, sym):
