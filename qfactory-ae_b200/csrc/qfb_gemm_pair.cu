@@ -183,16 +183,26 @@ struct PairTile {
       put(c, s);
     }
   }
-  // how many pieces have arrived (their sums are visible to the warp); called by whole warps
+  // How many pieces have arrived (their sums are visible to the warp); called by whole warps.  Lane 0 acquires; the
+  // barrier hands what it has seen to the other lanes, which a shuffle alone would not.
   __device__ __forceinline__ unsigned arrived() const {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
+    unsigned v = 0;
+    if (lane == 0) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
+    __syncwarp();
     return __shfl_sync(0xffffffffu, v, 0);
   }
   __device__ __forceinline__ unsigned arrive_lane() const { return atomicAdd(ctr, 1u); }
+  // the warp's sums are out (every lane's, by the barrier and lane 0's fence after it), and those of the pieces that
+  // arrived before are visible to every lane
   __device__ __forceinline__ unsigned arrive() const {
     unsigned prev = 0;
-    if (lane == 0) prev = arrive_lane();
+    __syncwarp();
+    if (lane == 0) {
+      __threadfence();
+      prev = arrive_lane();
+      __threadfence();
+    }
+    __syncwarp();
     return __shfl_sync(0xffffffffu, prev, 0);
   }
   __device__ __forceinline__ void reset_lane() const { *ctr = 0u; }
@@ -439,10 +449,7 @@ qgemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         tl.reset();
       } else {
         tl.publish(0, 32);
-        __threadfence();
-        __syncwarp();
         if (tl.arrive() == (unsigned)(tl.pieces - 1)) {
-          __threadfence();
           tl.sum(0, 32, false);
           tl.reset();
         }
