@@ -146,7 +146,7 @@ def test_outputs_ranks_strides_and_streams():
     for lead in ((), (1,), (2, 3), (3, 1, 2), (1, 6)):
         xr = x[0] if lead == () else x.reshape(*lead, 512) if torch.Size(lead).numel() == 6 else x[:1]
         y = layer(xr)
-        assert y.shape == (*xr.shape[:-1], 256) and torch.equal(y.reshape(-1, 256), want[: y.numel() // 256])
+        assert y.shape == (*xr.shape[:-1], 256) and torch.equal(y.reshape(-1, 256), layer(xr.reshape(-1, 512)))
     wide = torch.randn(6, 1024, device="cuda").half()
     wide[:, ::2] = x
     assert torch.equal(layer(wide[:, ::2]), want) and torch.equal(layer(x.t().contiguous().t()), want)
@@ -159,6 +159,7 @@ def test_outputs_ranks_strides_and_streams():
     for bad in (x.float(), x[:, :256], x.cpu(), torch.empty(0, 512, dtype=torch.float16, device="cuda")):
         with pytest.raises((AssertionError, RuntimeError)):
             layer(bad)
+    out = torch.empty_like(want)
     for bad in (out[:5], out.float(), torch.empty(256, 6, dtype=torch.float16, device="cuda").t()):
         with pytest.raises(AssertionError):
             layer(x, bad)
@@ -182,7 +183,7 @@ def test_the_fused_activation_gives_the_shape_of_the_rows(m):
 def test_flags_and_workspace_changed_after_the_first_call():
     from qfactory import _native
 
-    layer, x = _layer(m=24)
+    layer, x = _layer(m=24, k=4096)
     want = layer(x)
     assert _native.last_launch()["kernel"] == 2
     layer.flags = _native.FLAG_FORCE_SIMT
