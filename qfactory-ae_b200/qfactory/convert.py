@@ -31,11 +31,11 @@ def _check_scale(K, N, GS, scale):
     assert scale.dtype == torch.float16
 
 
-def _check_zero(K, N, GS, zero, nbits):
+def _check_zero(K, N, GS, zero, nbits, in_kernel):
     assert zero.shape == (K // GS, N)
     assert zero.dtype == torch.int32
-    if zero.is_cuda:
-        return
+    if in_kernel:
+        return   # as in _check_weight: the packing kernel goes where the codes are
     lo, hi = torch.aminmax(zero)
     assert lo >= 0 and hi < 2 ** nbits, "zero-points out of range"
 
@@ -157,7 +157,7 @@ def convert_params(args, params):
     _check_weight(K, N, weight, NBITS)
     _check_scale(K, N, GS, scale)
     if zero is not None:
-        _check_zero(K, N, GS, zero, NBITS)
+        _check_zero(K, N, GS, zero, NBITS, weight.is_cuda and zero.is_cuda)
     if weight.is_cuda:
         return _pack_native(K, N, NBITS, GS, weight, scale, zero, lay)
     if frag:

@@ -69,6 +69,8 @@ def test_values_out_of_range_are_reported():
             convert_params(args, (q2.cuda(), s.cuda(), z.cuda()))
         with pytest.raises(AssertionError, match="zero"):
             convert_params(args, (q.cuda(), s.cuda(), z2.cuda()))
+        with pytest.raises(AssertionError, match="zero"):   # codes on the CPU, zero points on the GPU
+            convert_params(args, (q, s, z2.cuda()))
     with pytest.raises(AssertionError, match="zero"):   # a group far below zero has a zero point no code can hold
         QLinear.from_float(torch.full((K, N), -3.0).half().cuda() + torch.rand(K, N).half().cuda(), 4, group)
 
