@@ -44,6 +44,13 @@ class _PackedLinear(torch.nn.Module):
         self.register_buffer("s", s)
         self.register_buffer("z", z)
 
+    def __setstate__(self, state):
+        super().__setstate__(state)
+        d = self.__dict__   # (a module pickled when these were plain attributes, and before there was a call object)
+        d.setdefault("_flags", d.pop("flags", 0))
+        d.setdefault("_ws_size", d.pop("_ws_bytes", 0))
+        d.setdefault("_native_call", None)
+
     # -- native plumbing ---------------------------------------------------
     @property
     def _ws(self):

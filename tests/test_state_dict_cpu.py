@@ -25,3 +25,23 @@ def test_state_dict_round_trip_keeps_the_bytes():
     b = QLinear.empty(1, 256, 128, 4, 128, False, device="cpu", layout="fragment")
     b.load_state_dict(a.state_dict())
     assert torch.equal(a.w, b.w) and b.packed_layout == layout.LAYOUT_FRAGMENT
+
+
+def test_modules_pickled_by_an_earlier_version_load():
+    import copy
+    import pickle
+
+    from qfactory import QLinear
+
+    layer = QLinear.empty(4, 256, 128, 4, 128, False, device="cpu")
+    old = dict(layer.__dict__)
+    for name in ("_native_call", "_flags", "_ws_size"):
+        del old[name]
+    old.update(flags=1, _ws_bytes=0)   # plain attributes then
+    revived = type(layer).__new__(type(layer))
+    revived.__setstate__(old)
+    assert revived.flags == 1 and revived._ws_bytes == 0 and revived._native_call is None
+    revived.flags = 2
+    for again in (pickle.loads(pickle.dumps(revived)), copy.deepcopy(revived)):
+        assert again.flags == 2 and again._native_call is None and again._ws_bytes == 0
+        assert again.w.equal(layer.w)
