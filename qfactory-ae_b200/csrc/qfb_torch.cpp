@@ -44,7 +44,8 @@ struct Abi {
   attention_rope_fn attention_rope;
 } abi = {};
 
-// what a native call of one layer needs; `hold` keeps the packed tensors and the workspace alive
+// what a native call of one layer needs; `hold` keeps the packed tensors and the workspace alive (a new workspace comes
+// with a new tuple)
 struct LayerCall {
   PyObject_HEAD
   qfb_layer desc;
@@ -118,10 +119,15 @@ PyObject* run_linear(LayerCall* L, PyObject* xo, PyObject* outo, bool fused) {
   const void* xp = x->data_ptr();
   void *yp = y.mutable_data_ptr(), *st = stream_of(L->device);
   const linear_fn fn = fused ? abi.linear_silu_mul : abi.linear;
+  // (read, and held, while no other thread can change them)
+  void* const ws = L->ws;
+  const size_t ws_bytes = (size_t)L->ws_bytes;
+  const unsigned flags = L->flags;
+  const THPObjectPtr hold(Py_XNewRef(L->hold));
   int status;
   {
     WithoutGil released;  // a launch waits where the stream's queue is full
-    status = fn(&L->desc, xp, (int)rows, yp, L->ws, (size_t)L->ws_bytes, L->flags, st);
+    status = fn(&L->desc, xp, (int)rows, yp, ws, ws_bytes, flags, st);
   }
   if (outo && outo != Py_None && status == 0) {
     Py_INCREF(outo);
@@ -174,6 +180,7 @@ PyMethodDef layer_methods[] = {
     {nullptr, nullptr, 0, nullptr}};
 PyMemberDef layer_members[] = {{"flags", T_UINT, offsetof(LayerCall, flags), 0, "QFB_FLAG_* of every call"},
                                {"ws_ptr", T_ULONGLONG, offsetof(LayerCall, ws), 0, "workspace address"},
+                               {"hold", T_OBJECT, offsetof(LayerCall, hold), 0, "what the pointers point into: (w, s, z, workspace)"},
                                {"ws_bytes", T_ULONGLONG, offsetof(LayerCall, ws_bytes), 0, "workspace size"},
                                {nullptr, 0, 0, 0, nullptr}};
 PyTypeObject LayerType = {PyVarObject_HEAD_INIT(nullptr, 0)};

@@ -61,8 +61,10 @@ class _PackedLinear(torch.nn.Module):
         # the workspace pointer handed to the hot call follows the tensor
         self._ws_tensor = t
         self._ws_ptr = t.data_ptr() if t is not None else None
-        if self._native_call is not None:
-            self._native_call.ws_ptr = self._ws_ptr or 0
+        nc = self._native_call
+        if nc is not None:
+            nc.ws_ptr = self._ws_ptr or 0
+            nc.hold = (*nc.hold[:3], t)
 
     @property
     def _ws_bytes(self):
@@ -106,7 +108,8 @@ class _PackedLinear(torch.nn.Module):
         silu_rows = (8 if self.n_bits == 3 else 16) if self.packed_layout == layout.LAYOUT_FRAGMENT else 0
         self._native_call = _native.torch_module().LayerCall(
             d.qweight or 0, d.scales or 0, d.zeros or 0, d.n, d.k, d.bits, d.group_size, d.layout, self._ws_ptr, nbytes,
-            self._flags, silu_rows, self.w.get_device(), (self.w, self.s, self.z))
+            self._flags, silu_rows, self.w.get_device(),
+            (self.w, self.s, self.z, self._ws))
 
     # -- the packed layout travels with the checkpoint ------------------------
     def get_extra_state(self):

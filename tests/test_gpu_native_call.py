@@ -193,6 +193,7 @@ def test_flags_and_workspace_changed_after_the_first_call():
     layer._ws = torch.zeros_like(layer._ws)
     assert torch.equal(layer(x), want)
     held = layer._ws
+    assert layer._native_call.hold == (layer.w, layer.s, layer.z, held) and layer._native_call.ws_ptr == held.data_ptr()
     layer._ws_bytes = 0
     with pytest.raises(_native.NativeError):   # a split without room for its partial sums
         layer(x)
