@@ -6,12 +6,14 @@ Compiles every csrc/*.cu with nvcc (one process per file, in parallel) and links
 lib/libqfactory_b200.so.  The library only depends on the statically linked CUDA
 runtime, so it loads on a machine without a GPU (calls then fail with a CUDA error).
 csrc/qfb_torch.cpp, the CPython module that calls the library on torch tensors, is
-compiled with g++ against the installed torch's headers into lib/_qfb_torch.so.
-A source newer than its library triggers a rebuild.
+compiled with g++ against the installed torch's headers into lib/_qfb_torch.so; without
+torch only the library is built, which is all that the C ABI needs.
+A source newer than its library triggers a rebuild, and another torch or Python one of the module.
 """
 from __future__ import annotations
 
 import glob
+import importlib.metadata
 import os
 import subprocess
 import sys
@@ -25,6 +27,7 @@ LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libqfactory_b200.so")
 TORCH_SRC = os.path.join(CSRC, "qfb_torch.cpp")
 TORCH_LIB = os.path.join(LIB_DIR, "_qfb_torch.so")
+TORCH_FOR = os.path.join(OBJ, "_qfb_torch.for")   # the torch and the Python it was built against
 HEADER = os.path.join(os.path.dirname(HERE), "include", "qfactory_b200.h")
 
 NVCC_FLAGS = [
@@ -57,13 +60,39 @@ def is_stale() -> bool:
     return any(os.path.getmtime(d) > t for d in _deps())
 
 
-def build_torch_module(force: bool = False, verbose: bool = False) -> str:
-    if not force and os.path.exists(TORCH_LIB) and all(
-            os.path.getmtime(d) <= os.path.getmtime(TORCH_LIB) for d in (TORCH_SRC, HEADER)):
+def _torch_version() -> str | None:
+    try:   # (without importing it, which takes seconds)
+        return importlib.metadata.version("torch")
+    except importlib.metadata.PackageNotFoundError:
+        return None
+
+
+def torch_module_is_stale(version: str) -> bool:
+    """Older than its sources, or built for another torch or Python than the ones here."""
+    if not os.path.exists(TORCH_LIB) or any(os.path.getmtime(d) > os.path.getmtime(TORCH_LIB) for d in (TORCH_SRC, HEADER)):
+        return True
+    try:
+        with open(TORCH_FOR) as f:
+            return f.read() != _built_for(version)
+    except OSError:
+        return True
+
+
+def _built_for(version: str) -> str:
+    return f"torch {version}, {sysconfig.get_config_var('SOABI')}"
+
+
+def build_torch_module(force: bool = False, verbose: bool = False) -> str | None:
+    version = _torch_version()
+    if version is None:
+        sys.stderr.write("torch is not installed: the library is built, the module for torch tensors is not\n")
+        return None
+    if not force and not torch_module_is_stale(version):
         return TORCH_LIB
     import torch
 
     os.makedirs(LIB_DIR, exist_ok=True)
+    os.makedirs(OBJ, exist_ok=True)
     root = os.path.dirname(torch.__file__)
     cuda_inc = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
     tmp = TORCH_LIB + ".tmp"
@@ -77,11 +106,18 @@ def build_torch_module(force: bool = False, verbose: bool = False) -> str:
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed on {TORCH_SRC}")
     os.replace(tmp, TORCH_LIB)
+    with open(TORCH_FOR, "w") as f:
+        f.write(_built_for(version))
     return TORCH_LIB
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
+    lib = build_library(force, verbose)
     build_torch_module(force, verbose)
+    return lib
+
+
+def build_library(force: bool = False, verbose: bool = False) -> str:
     if not force and not is_stale():
         return LIB
     os.makedirs(OBJ, exist_ok=True)
