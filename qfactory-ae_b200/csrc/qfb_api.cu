@@ -380,7 +380,7 @@ static int choose_kernel(const LayerView& v, int m, unsigned flags) {
   if (!tc_supported(v)) return 1;
   // K an odd multiple of 64: the CUDA-core kernel takes 8 rows a pass and reads the weights again for every 8 more
   // ((3000,2752) at 37 rows: 79 us against 12)
-  if (v.k % 128 != 0) return m > kMaxSimtRows ? 2 : 1;
+  if (v.k % 128 != 0) return m > kMaxSimtRows && ((flags & QFB_FLAG_FORCE_TENSOR) || m >= g_tc_min_m) ? 2 : 1;
   if (flags & QFB_FLAG_FORCE_TENSOR) return 2;
   if (m >= g_tc_min_m) return 2;
   // a single activation row: the CUDA-core kernel wins while the packed weight is small
@@ -436,7 +436,7 @@ static int run_gemv(const LayerView& v, const __half* x, int m, __half* y, void*
     p.max_units_per_cta = (v.units + pl.split - 1) / pl.split;
     p.units_per_kway = (p.max_units_per_cta + pl.kways - 1) / pl.kways;
     p.zconst = v.zconst;
-  p.early = (flags & QFB_FLAG_PDL) ? 1 : 0;
+    p.early = (flags & QFB_FLAG_PDL) ? 1 : 0;
     p.partial = nullptr;
     p.counters = nullptr;
     if (pl.split > 1) {
