@@ -156,7 +156,8 @@ def test_outputs_ranks_strides_and_streams():
         y = layer(x)
     side.synchronize()
     assert torch.equal(y, want)
-    for bad in (x.float(), x[:, :256], x.cpu(), torch.empty(0, 512, dtype=torch.float16, device="cuda")):
+    assert layer(x[:0]).shape == (0, 256) and layer(x[:0].view(2, 0, 512)).shape == (2, 0, 256)
+    for bad in (x.float(), x[:, :256], x.cpu()):
         with pytest.raises((AssertionError, RuntimeError)):
             layer(bad)
     out = torch.empty_like(want)

@@ -24,6 +24,18 @@ CASES = [
 ]
 
 
+def _is_pair_launch(m, n, k, cut):
+    """The launch as it is planned for CTA pairs.  (The single-CTA kernel has a CTA for every row tile and batch tile, or
+    for every part of one, and batch tiles of 64, 128 or 256 columns.)"""
+    slots = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    mtiles = -(-m // 256)
+    nb = -(-(-(-m // mtiles)) // 32) * 32
+    units = (-(-n // 128) + 1) // 2 * mtiles
+    pairs = min(slots, units * -(-k // 128) // 16) if cut else min(slots, units)
+    info = _native.last_launch()
+    assert info == {"kernel": 2, "grid_x": 2 * pairs, "grid_y": 2 if cut else 1, "block": 768, "smem": nb}, info
+
+
 @pytest.mark.parametrize("m,n,k,bits,group,sym,layout,cut", CASES)
 def test_against_double_precision(m, n, k, bits, group, sym, layout, cut):
     g = torch.Generator(device="cuda").manual_seed(m + n + k)
@@ -41,8 +53,7 @@ def test_against_double_precision(m, n, k, bits, group, sym, layout, cut):
         w = s.repeat_interleave(group, 0) * (codes - zz.repeat_interleave(group, 0)).half()
     y = layer(x)
     torch.cuda.synchronize()
-    info = _native.last_launch()
-    assert info["block"] == 768 and info["smem"] % 32 == 0 and info["grid_y"] == (2 if cut else 1), info
+    _is_pair_launch(m, n, k, cut)
     st = ctypes.c_uint(0)
     assert _native.lib().qfb_read_status(layer._ws.data_ptr(), None, ctypes.byref(st)) == 0 and st.value == 0
     for c0 in range(0, n, 4096):
@@ -62,10 +73,10 @@ def test_without_room_for_partial_sums_units_run_whole():
     layer = QLinear.init(m, k, n, 4, codes, 128, s, None)
     x = torch.randn(m, k, generator=g, device="cuda").half()
     y = layer(x)
-    assert _native.last_launch()["grid_y"] == 2
+    _is_pair_launch(m, n, k, True)
     layer._ws_bytes = 1 << 20
     y2 = layer(x)
-    assert _native.last_launch()["grid_y"] == 1
+    _is_pair_launch(m, n, k, False)
     # fp32 sums in another order, both rounded to fp16
     bound = 2.0 ** -9 * y.float().abs() + k / 16 * 2.0 ** -22 * y.float().abs().max()
     assert bool(((y.float() - y2.float()).abs() <= bound).all())
@@ -85,3 +96,31 @@ def test_split_tiles_of_33_to_64_rows_without_a_workspace():
     assert _native.last_launch()["grid_y"] == 1
     bound = 2.0 ** -9 * y.float().abs() + k / 16 * 2.0 ** -22 * y.float().abs().max()
     assert bool(((y.float() - y2.float()).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("m,n,k,layout,cut", [(200, 8192, 8192, "fragment", True), (300, 18944, 2560, "tile", False)])
+def test_a_wait_that_runs_out_abandons_the_launch_in_both_ctas(m, n, k, layout, cut):
+    """The test flag of test_gpu_bounded_waits.py: 16 bytes that never come on the first weight barrier of every CTA, waits
+    of about 100 us.  Nothing is stored, the status word is raised, and the layer then runs as before: its counters are
+    untouched and tensor memory is free in both CTAs of every pair."""
+    g = torch.Generator(device="cuda").manual_seed(7)
+    codes = torch.randint(0, 16, (k, n), generator=g, dtype=torch.int32, device="cuda")
+    s = (torch.rand(k // 128, n, generator=g, device="cuda") * 0.018 + 0.002).half()
+    layer = QLinear.init(m, k, n, 4, codes, 128, s, None, layout=layout)
+    x = torch.randn(m, k, generator=g, device="cuda").half()
+    st = ctypes.c_uint(0)
+    status = lambda: (_native.lib().qfb_read_status(layer._ws.data_ptr(), None, ctypes.byref(st)), st.value)  # noqa: E731
+    want = layer(x)
+    _is_pair_launch(m, n, k, cut)
+    assert status() == (0, 0)
+    out = torch.full_like(want, 7.0)
+    layer.flags = _native.FLAG_TEST_STALLED_WAIT
+    layer(x, out)
+    torch.cuda.synchronize()
+    _is_pair_launch(m, n, k, cut)
+    assert status() == (8, 1) and bool((out == 7.0).all())   # QFB_ERR_DEVICE_FLAG
+    layer.flags = 0
+    _native.check(_native.lib().qfb_workspace_init(layer._ws.data_ptr(), layer._ws_bytes, torch.cuda.current_stream().cuda_stream))
+    for _ in range(3):
+        assert torch.equal(layer(x), want)
+    assert status() == (0, 0)
