@@ -76,38 +76,64 @@ struct TcCfg {
   static_assert(kDBase + (POST ? kRing * NB : kIssuers * NB) <= kTmemCols, "tensor memory over-subscribed");
 };
 
-// Sum of the split-K partials of one warp's 32 rows (lane = row) over all S splits, in split order,
-// rounded to fp16 into y, for the tiles with per-stage accumulators.  base0 -> partial of split 0, batch column 0, this
-// lane's row; `sstride` floats between splits, `cstride` between batch columns; ydst -> y[first batch row][this lane's
-// output feature], `ystride` halfs between batch rows; `cols` = valid batch columns.  8 columns of four splits are in
-// flight per round (a column at a time cost one round trip per column).
+// Sum of the split-K partials of one warp's 32 rows over all S splits, in split order, rounded to fp16 into y, for the
+// tiles with per-stage accumulators.  part -> partial of split 0, batch column 0, the warp's first row; `sstride` floats
+// between splits, `cstride` between batch columns (both multiples of 128); y -> y[first batch row][the warp's first
+// output feature], `ystride` halfs between batch rows; `cols` valid batch columns, `rows` valid rows.
+// A lane sums four rows of every fourth column: 16 columns of two splits, eight 16-byte loads a lane, are in flight per
+// round.  With a row per lane and 32 loads of 4 bytes in flight this build's 64 registers did not suffice: it spilled and
+// waited in between.  Measured, that -> this, (4096,11008), 9 splits: 16 rows (tile layout) 30.0 -> 15.8 us, 32 rows 31.2 ->
+// 20.9; 8-bit (8192,8192) at 24 rows 27.6 -> 23.9 (launches one after the other from a graph).
 template <int NB>
-__device__ __forceinline__ void splitk_reduce(const float* base0, size_t sstride, size_t cstride, int S, int cols,
-                                              bool row_ok, __half* ydst, size_t ystride) {
-  constexpr int CW = 8, SPB = 4;
+__device__ __forceinline__ void splitk_reduce(const float* part, uint32_t sstride, uint32_t cstride, int S, int cols, int rows,
+                                              __half* y, size_t ystride, int lane) {
+  // (opaque: from strides it knows to be products of launch constants the compiler precomputes more addresses than the
+  // build has registers for)
+  asm("" : "+r"(sstride), "+r"(cstride));
+  const int r = (lane & 7) * 4, cg = lane >> 3;
+  const bool vec = rows >= r + 4 && ystride % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & 7u) == 0;
 #pragma unroll 1
-  for (int c0 = 0; c0 < NB; c0 += CW) {
-    if (c0 >= cols) break;
-    float sum[CW];
+  for (int c0 = cg; c0 - cg < NB && c0 - cg < cols; c0 += 16) {
+    float4 sum[4];
 #pragma unroll
-    for (int j = 0; j < CW; ++j) sum[j] = 0.f;
+    for (int j = 0; j < 4; ++j) sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float* b = part + (size_t)(c0 * cstride + r);
 #pragma unroll 1
-    for (int sp = 0; sp < S; sp += SPB) {
-      float t[SPB][CW];
+    for (int sp = 0; sp < S; sp += 2, b += 2 * (size_t)sstride) {
+      float4 t[2][4];
 #pragma unroll
-      for (int u = 0; u < SPB; ++u)
+      for (int u = 0; u < 2; ++u)
 #pragma unroll
-        for (int j = 0; j < CW; ++j)
-          t[u][j] = (sp + u < S && c0 + j < cols) ? __ldcg(base0 + (size_t)(sp + u) * sstride + (size_t)(c0 + j) * cstride) : 0.f;
+        for (int j = 0; j < 4; ++j)
+          t[u][j] = (sp + u < S && c0 + 4 * j < cols) ? __ldcg(reinterpret_cast<const float4*>(b + u * sstride + 4 * j * cstride))
+                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int u = 0; u < SPB; ++u)
+      for (int u = 0; u < 2; ++u)
+        if (sp + u < S) {
 #pragma unroll
-        for (int j = 0; j < CW; ++j)
-          if (sp + u < S) sum[j] += t[u][j];
+          for (int j = 0; j < 4; ++j) {
+            sum[j].x += t[u][j].x;
+            sum[j].y += t[u][j].y;
+            sum[j].z += t[u][j].z;
+            sum[j].w += t[u][j].w;
+          }
+        }
     }
 #pragma unroll
-    for (int j = 0; j < CW; ++j)
-      if (c0 + j < cols && row_ok) ydst[(size_t)(c0 + j) * ystride] = __float2half_rn(sum[j]);
+    for (int j = 0; j < 4; ++j) {
+      const int c = c0 + 4 * j;
+      if (c >= cols) continue;
+      __half* dst = y + (size_t)c * ystride + r;
+      const __half2 lo = __floats2half2_rn(sum[j].x, sum[j].y), hi = __floats2half2_rn(sum[j].z, sum[j].w);
+      if (vec) {
+        *reinterpret_cast<uint2*>(dst) = make_uint2(as_u32(lo), as_u32(hi));
+      } else {
+        if (r < rows) dst[0] = __low2half(lo);
+        if (r + 1 < rows) dst[1] = __high2half(lo);
+        if (r + 2 < rows) dst[2] = __low2half(hi);
+        if (r + 3 < rows) dst[3] = __high2half(hi);
+      }
+    }
   }
 }
 
@@ -380,8 +406,9 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
         prev = __shfl_sync(0xffffffffu, prev, 0);
         if (prev != (unsigned)(S - 1)) return;
         __threadfence();
-        splitk_reduce<NB>(p.partial + (size_t)m0 * p.npad + n, (size_t)p.m * p.npad, (size_t)p.npad, S, p.m - m0, n < p.n,
-                          p.y + (size_t)m0 * p.n + n, (size_t)p.n);
+        const int n0 = n - lane;
+        splitk_reduce<NB>(p.partial + (size_t)m0 * p.npad + n0, (uint32_t)p.m * p.npad, (uint32_t)p.npad, S, p.m - m0,
+                          p.n - n0, p.y + (size_t)m0 * p.n + n0, (size_t)p.n, lane);
         if (lane == 0) *ctr = 0u;
       };
       float acc[NB];
