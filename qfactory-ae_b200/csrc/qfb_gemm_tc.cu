@@ -219,7 +219,11 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
   const uint32_t tmem_base = tmem_holder;
   volatile int* abortp = &abort_flag;
   const long long wait_limit = p.stall_test ? 200000LL : kWaitLimitCycles;
-  grid_launch_dependents();
+  // Builds with two CTAs per SM let the next kernel in only when their stages are done: its CTAs would fill the slots this
+  // grid leaves free, two on some SMs beside others with none, and stay there.  Launches in a row, at once -> late:
+  // (12288,4096) at 24 rows, 96 CTAs, 29.5 -> 24.5 us; (25600,8192) at 33 rows, 252 CTAs, 61.2 -> 47.8; (28672,8192) at 64, 224
+  // CTAs, 63.2 -> 62.0; with all slots taken no difference.  (A layer that reads early gains more from being in early.)
+  if (p.early || !Cfg::kTwoPerSM) grid_launch_dependents();
   if (!p.early) grid_dependency_wait();
 
   const bool has_z = ASYM || p.qz != nullptr;
@@ -452,6 +456,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
         }
         if (++r == R) { r = 0; phr ^= 1; }
       }
+      if (!p.early) grid_launch_dependents();
       if (ok) {
         grid_dependency_wait();  // y and the workspace may still be in use by the preceding kernel
 #pragma unroll
@@ -469,6 +474,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (Cfg::kTwoPerSM && !p.early) grid_launch_dependents();
     if (!*abortp) {   // (an abandoned launch stores nothing)
       grid_dependency_wait();
       const int q = warp & 3, m0 = mtile * NB, n0 = tile * kTileRows + q * 32, n = n0 + lane;
