@@ -203,10 +203,11 @@ static TcPlan plan_tc(const LayerView& v, int m) {
                             m <= 128;
     pl.dg = g_tc_dg > 0 ? std::min(g_tc_dg, 2) : (two_per_sm ? 1 : 2);
     // More row tiles than SMs, two CTAs per SM: the tiles beyond a whole number per SM are cut along K, so that they do
-    // not cost a whole tile's time more on a few SMs ((57344,8192) at 128 rows, 448 tiles on 148 SMs: 143 -> 128.5 us;
-    // (28672,8192), 224 tiles: 75.9 -> 73.6)
+    // not cost a whole tile's time more on a few SMs ((57344,8192) at 128 rows, 448 tiles on 148 SMs: 143 -> 128.5 us).
+    // Only where their parts are no more than the SMs: beyond, the parts need a turn of their own ((32000,4096), 250
+    // tiles, 102 of them cut in two: 45.9 us at 64 rows and 55.6 at 128, whole 34.4 and 39.8).
     const int units = v.tiles * pl.mtiles, slots = num_sms(), rest = units % slots;
-    if (two_per_sm && pl.split == 1 && g_tc_split == 0 && rest > 0 && stages_of(v) >= 32) {
+    if (two_per_sm && pl.split == 1 && g_tc_split == 0 && rest > 0 && rest * 2 <= slots && stages_of(v) >= 32) {
       pl.tail_split = rest * 4 <= slots ? 4 : rest * 3 <= slots ? 3 : 2;
       pl.full_units = units - rest;
       pl.tail_units = rest;

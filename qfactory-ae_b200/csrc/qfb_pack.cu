@@ -374,11 +374,13 @@ cudaError_t launch_quantize(const __half* w, int k, int n, int bits, int group_s
 // ever reach memory.  One CTA owns the 128 rows of a tile and one run of k: a whole group, or two groups of 64.  Thread
 // (pair of rows c, quarter h) holds 32 k of its two rows of a 128-k block in registers, so a group of at most 128 is
 // read once; a longer one is read a second time (from L2) after its extremes are known.
-// (w - min) / span is computed as (w - min) * (1 / span), both operations rounded to fp32, then rounded to fp16.  That
-// equals the division's result in every case: with a = w - min and b = span in fp16 (11-bit significands) the product
-// is within 2^-23 (1 + 2^-25) of a / b, relative, while a / b stays more than that away from every midpoint m of two
-// fp16 values (12 bits): it is never equal to one, since m * b has at least 12 bits, and |a - m b| is at least one unit
-// against m b < 2^23 units.
+// (w - min) / span is computed as (w - min) * (1 / span), both operations rounded to fp32, then rounded to fp16.  Where
+// the quotient is a normal fp16 value that equals the division's result: with a = w - min and b = span in fp16 (11-bit
+// significands) the product is within 2^-23 (1 + 2^-25) of a / b, relative, while a / b stays more than that away from
+// every midpoint m of two neighbouring normal values (12 bits): it is never equal to one, since m * b has at least 12
+// bits, and |a - m b| is at least one unit against m b < 2^23 units.  A quotient below 2^-14 can come out one subnormal
+// step off (its midpoints have fewer bits); times at most 255 levels it is less than one either way, so that the code
+// is 0 and the zero point, which is that less one, is 0.
 // Instruction bound at about twice the memory time: (8192,28672) 4-bit, groups of 128, 182 us for 592 MB in and out.
 template <int BITS, bool FRAG>
 __global__ void __launch_bounds__(kPackThreads, 4) quantize_pack_kernel(const PackParams p, int run) {
