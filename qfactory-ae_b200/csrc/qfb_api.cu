@@ -281,8 +281,9 @@ static int run_tc(const LayerView& v, const __half* x, int m, __half* y, void* w
           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return QFB_ERR_CUDA;
+  // (read by the builds with kSwizzledStage only: not with per-stage accumulators)
   CUtensorMap tw = {};
-  if (v.layout == QFB_LAYOUT_FRAGMENT && (v.bits == 4 || v.bits == 8)) {
+  if (v.layout == QFB_LAYOUT_FRAGMENT && (v.bits == 4 || v.bits == 8) && !pl.post) {
     const cuuint64_t wdim[2] = {16, (cuuint64_t)v.npad * v.k * v.bits / 512};
     const cuuint64_t wstr[1] = {64};
     const cuuint32_t wbox[2] = {16, (cuuint32_t)(16 * v.bits)};
