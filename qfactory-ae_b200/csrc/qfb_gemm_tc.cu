@@ -70,6 +70,11 @@ struct TcCfg {
   static constexpr int kRingCap = kXStages < 6 ? kXStages : 6;   // never deeper than the activation ring
   static constexpr int kRing = kRingRaw > kRingCap ? kRingCap : kRingRaw;
   static constexpr int kDBase = kRing * kAColsPerSlot;
+  // What the CTA works on is not kept through the roles for the results, but worked out again: where two CTAs share an SM
+  // the decode loop needs every one of the 64 registers.  (28672,8192): 3 bits at 64 rows 95.8 -> 88.4 us, 4 bits at 128 rows
+  // 71.2 -> 69.4; not at 64 columns with the smaller decoders (4 bits at 64 rows 62.0 -> 66.4: the results' code spills)
+  // nor with one CTA per SM (no difference, and 1 us more where K is split).
+  static constexpr bool kRederive = kTwoPerSM && !POST && (NB > 64 || BITS == 3);
   static constexpr size_t kSmemBytes = 1024 + (size_t)kXStages * kXBytes + (size_t)kWStages * (kWBytes + kQBytes);
   static_assert(kWStages >= 2, "weight ring too shallow");
   static_assert(kRing >= 2, "need at least two tensor-memory slots");
@@ -137,6 +142,44 @@ __device__ __forceinline__ void splitk_reduce(const float* part, uint32_t sstrid
   }
 }
 
+// What a CTA works on.  Two grid shapes.  Uniform: grid (row tiles, batch tiles, K splits).  Tail-split (p.tail_split > 0,
+// one-dimensional grid): the first p.full_units CTAs own a whole (row tile, batch tile) unit each,
+// the remaining units (the last, partly filled wave of a launch) are cut into p.tail_split K ranges
+// of one CTA each, so that the tail costs a fraction of a wave.
+struct TcUnit {
+  int tile, mtile, split, S;   // K range `split` of the unit's S
+  int ctr;                     // index of the unit's arrival counters
+  int tail;                    // >= 0: this CTA writes compact partials of tail unit `tail`
+  int kb0, nkb;                // the range's first stage and how many it has
+};
+__device__ __forceinline__ TcUnit tc_unit(const TcParams& p, int cx, int cy, int cz) {
+  TcUnit u;
+  u.tile = cx;
+  u.mtile = cy;
+  u.split = cz;
+  u.S = gridDim.z;
+  u.ctr = cy * gridDim.x + cx;
+  u.tail = -1;
+  if (p.tail_split > 0) {
+    int unit = cx;
+    u.split = 0;
+    u.S = 1;
+    if (cx >= p.full_units) {
+      const int j = cx - p.full_units;
+      u.tail = j / p.tail_split;
+      unit = p.full_units + u.tail;
+      u.split = j - u.tail * p.tail_split;
+      u.S = p.tail_split;
+      u.ctr = u.tail;
+    }
+    u.tile = unit / p.mtiles;
+    u.mtile = unit - u.tile * p.mtiles;
+  }
+  u.kb0 = (int)(((long long)u.split * p.kblocks) / u.S);
+  u.nkb = (int)(((long long)(u.split + 1) * p.kblocks) / u.S) - u.kb0;
+  return u;
+}
+
 // FRAG = the layer is in the fragment layout (a build of its own: with both decoders behind a run-time branch in
 // the decode loop the compiler allots registers for the larger of the two)
 // ASYM = the layer has scales AND zero points (the common case; a build of its own for the same reason; used
@@ -157,32 +200,8 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
   __shared__ unsigned tail_seen[4];   // per 32 rows: K ranges that have arrived / this one is the last
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // Two grid shapes.  Uniform: grid (row tiles, batch tiles, K splits).  Tail-split (p.tail_split > 0,
-  // one-dimensional grid): the first p.full_units CTAs own a whole (row tile, batch tile) unit each,
-  // the remaining units (the last, partly filled wave of a launch) are cut into p.tail_split K ranges
-  // of one CTA each, so that the tail costs a fraction of a wave.
-  int tile = blockIdx.x, mtile = blockIdx.y, split = blockIdx.z, S = gridDim.z;
-  int unit_ctr = mtile * gridDim.x + tile;   // index of this unit's arrival counters
-  int tail_unit = -1;                        // >= 0: this CTA writes compact partials of tail unit `tail_unit`
-  if (p.tail_split > 0) {
-    const int c = blockIdx.x;
-    int unit = c;
-    split = 0;
-    S = 1;
-    if (c >= p.full_units) {
-      const int j = c - p.full_units;
-      tail_unit = j / p.tail_split;
-      unit = p.full_units + tail_unit;
-      split = j - tail_unit * p.tail_split;
-      S = p.tail_split;
-      unit_ctr = tail_unit;
-    }
-    tile = unit / p.mtiles;
-    mtile = unit - tile * p.mtiles;
-  }
-  const int kb0 = (int)(((long long)split * p.kblocks) / S);
-  const int kb1 = (int)(((long long)(split + 1) * p.kblocks) / S);
-  const int nkb = kb1 - kb0;
+  const TcUnit unit = tc_unit(p, blockIdx.x, blockIdx.y, blockIdx.z);
+  const int tile = unit.tile, mtile = unit.mtile, split = unit.split, S = unit.S, kb0 = unit.kb0, nkb = unit.nkb;
 
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gbase = smem_raw + (sbase - smem_u32(smem_raw));
@@ -405,7 +424,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
         __threadfence();
         __syncwarp();
         unsigned prev = 0;
-        unsigned* ctr = p.counters + (unit_ctr * 4 + q);
+        unsigned* ctr = p.counters + (unit.ctr * 4 + q);
         if (lane == 0) prev = atomicAdd(ctr, 1u);
         prev = __shfl_sync(0xffffffffu, prev, 0);
         if (prev != (unsigned)(S - 1)) return;
@@ -477,12 +496,19 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
     if (Cfg::kTwoPerSM && !p.early) grid_launch_dependents();
     if (!*abortp) {   // (an abandoned launch stores nothing)
       grid_dependency_wait();
-      const int q = warp & 3, m0 = mtile * NB, n0 = tile * kTileRows + q * 32, n = n0 + lane;
+      // (kRederive: worked out again from what the hardware knows)
+      int cx = blockIdx.x, cy = blockIdx.y, cz = blockIdx.z, tid = threadIdx.x;
+      if constexpr (Cfg::kRederive)
+        asm volatile("mov.u32 %0, %%ctaid.x;\n\tmov.u32 %1, %%ctaid.y;\n\tmov.u32 %2, %%ctaid.z;\n\tmov.u32 %3, %%tid.x;"
+                     : "=r"(cx), "=r"(cy), "=r"(cz), "=r"(tid));
+      const TcUnit u = Cfg::kRederive ? tc_unit(p, cx, cy, cz) : unit;
+      const int warp = tid >> 5, lane = tid & 31, split = u.split, S = u.S, tail_unit = u.tail;
+      const int q = warp & 3, m0 = u.mtile * NB, n0 = u.tile * kTileRows + q * 32, n = n0 + lane;
       const int cols = min(NB, p.m - m0);
       const int c0 = (warp >> 2) * 16;
       constexpr int kStep = Cfg::kThreads / 128 * 16;
-      const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + Cfg::kDBase;
-      const bool two = Cfg::kIssuers == 2 && nkb >= 2;  // the second accumulator holds something
+      const uint32_t acc = (Cfg::kRederive ? *static_cast<volatile uint32_t*>(&tmem_holder) : tmem_base) + ((uint32_t)(q * 32) << 16) + Cfg::kDBase;
+      const bool two = Cfg::kIssuers == 2 && u.nkb >= 2;  // the second accumulator holds something
       const bool vec = n0 + 32 <= p.n && p.n % 8 == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15u) == 0;
       __half* y = p.y + (size_t)m0 * p.n + n0;
       auto load16 = [&](int c, float (&f)[16]) {
@@ -531,7 +557,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
       } else {
         // the last range to arrive, per 32 rows, sums them all; one that finds the others there when it comes needs
         // no partial sums of its own in memory
-        unsigned* ctr = p.counters + (unit_ctr * 4 + q);
+        unsigned* ctr = p.counters + (u.ctr * 4 + q);
         if (warp < 4 && lane == 0) {
           unsigned seen;
           asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(ctr) : "memory");
@@ -586,7 +612,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
   }
   if (warp == 2) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, Cfg::kTmemCols);
+    tmem_dealloc(Cfg::kRederive ? *static_cast<volatile uint32_t*>(&tmem_holder) : tmem_base, Cfg::kTmemCols);
   }
 }
 
