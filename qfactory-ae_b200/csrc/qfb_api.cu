@@ -465,7 +465,7 @@ static int run_gemv(const LayerView& v, const __half* x, int m, __half* y, void*
 // warps of the mma.sync GEMV an SM holds: 16 at 128 registers per thread, 20 at 96 (CTAs of up to
 // kMmaSmallBlock threads)
 static int mma_warps_per_sm(int block) { return block <= kMmaSmallBlock ? 20 : 16; }
-struct MmaPlan { int nt, split, kways, cluster, recv_offset; size_t smem; };
+struct MmaPlan { int nt, split, kways, cluster, recv_offset; bool tight; size_t smem; };
 
 // most splits through the workspace (its size follows from this bound)
 static int mma_split_cap(int tiles, int batches) {
@@ -510,7 +510,7 @@ static MmaPlan plan_mma_search(int tiles, int k, int rows, bool seg64, int bits,
   const int cap_ws = mma_split_cap(tiles, batches);
   const int cap = std::max(cap_ws, g_mma_cluster ? mma_cluster_split_cap(tiles, batches, 32 * wpk) : 1);
   const size_t smem_max = 100 * 1024;
-  int best_s = cap_ws, best_kw = 1, best_cl = 0;
+  int best_s = cap_ws, best_kw = 1, best_cl = 0, best_fit = 0;
   double best_cost = 1e30;
   for (int kw = kways_max; kw >= 1; kw >>= 1) {
     if (g_tune_kways > 0 && kw != std::min(g_tune_kways, kways_max)) continue;
@@ -534,13 +534,14 @@ static MmaPlan plan_mma_search(int tiles, int k, int rows, bool seg64, int bits,
         if (fit > 0) {
           const int waves = (tiles + fit - 1) / fit;
           const double cost = (double)waves * (per_kway + 1.5) + base + 0.02 * rows * s;
-          if (cost < best_cost) { best_cost = cost; best_s = s; best_kw = kw; best_cl = 1; }
+          if (cost < best_cost) { best_cost = cost; best_s = s; best_kw = kw; best_cl = 1; best_fit = fit; }
         }
       }
     }
   }
   pl.split = best_s;
   pl.cluster = best_cl;
+  pl.tight = best_cl && tiles <= best_fit && tiles * 1000LL > best_fit * 985LL;
   const int bpc = (batches + best_s - 1) / best_s;
   // a power of two (the kernel splits a CTA's range among the k-ways with a shift), no more than the batches of a CTA
   pl.kways = best_kw;
@@ -641,6 +642,11 @@ static int run_mma(const LayerView& v, const __half* x, int m, __half* y, void* 
       p.counters = reinterpret_cast<unsigned*>(static_cast<char*>(workspace) + kHeaderBytes);
       p.partial = reinterpret_cast<float*>(static_cast<char*>(workspace) + off);
     }
+    // Clusters that fill every place there is for them wait until the preceding grid has gone: let in early, they find
+    // the places it leaves one by one, some of which then lie in two GPCs and serve no cluster.  us with the overlap -> without,
+    // (7168,5120) at 8 rows, 56 clusters in 56 places, 8.4 -> 7.6; (18176,4096) 8-bit, 142 in 142, 17.9 -> 15.3; (9000,3072)
+    // 8-bit at 16, 71 in 71, 11.1 -> 9.5; with 172 in 175 or fewer the overlap gains ((22016,4096) at one row 11.8 -> 10.1).
+    p.overlap = p.early || !p.cluster || !pl.tight;
     const dim3 grid(pl.split, v.tiles);
     const int block = 32 * (kTileRows / mma_rows_per_warp(v.bits, pl.nt)) * pl.kways;
     tl_last_launch[0] = 3;

@@ -842,7 +842,7 @@ static cudaError_t launch_cfg(const MmaParams& p, dim3 grid, int block, size_t s
   cudaLaunchAttribute attr[2];
   int na = 1;
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[0].val.programmaticStreamSerializationAllowed = p.overlap;
   if (p.cluster) {  // the K splits of one tile form a cluster
     attr[na].id = cudaLaunchAttributeClusterDimension;
     attr[na].val.clusterDim.x = grid.x;

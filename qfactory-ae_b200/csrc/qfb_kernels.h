@@ -26,8 +26,8 @@ struct GemvParams {
   int early;             // weights, scales and zeros may be read before the preceding kernel has finished
 };
 
-// All linear kernels are launched with programmatic stream serialisation: the launch and the set-up of their CTAs
-// overlap the end of the preceding kernel.  What may be read before griddepcontrol.wait is the caller's to say
+// The linear kernels are launched with programmatic stream serialisation (for an exception see run_mma): the launch and
+// the set-up of their CTAs overlap the end of the preceding kernel.  What may be read before griddepcontrol.wait is the caller's to say
 // (QFB_FLAG_PDL -> `early`): without it the wait comes before the first read of anything.  Measured, launches one
 // after the other from the host, plain stream order -> wait first -> early reads: 3-bit (8192,8192) at 4 rows 12.3 ->
 // 10.3 -> 10.0 us, the four linears of a 7B layer at one row 43.6 -> 33.2 -> 32.9 us.
@@ -87,6 +87,7 @@ struct MmaParams {
   int batches_div, batches_mod;  // batches / S and batches % S: split s owns batches_div (+1 if s < batches_mod)
   uint32_t zconst;
   int early;             // weights, scales and zeros may be read before the preceding kernel has finished
+  int overlap;           // launched with programmatic stream serialisation
   int cluster;           // 1: the S splits of a tile are one thread-block cluster and reduce in shared memory
   int recv_offset;       // byte offset of the cluster reduction's receive buffer in dynamic shared memory
   int quads_per_owner;   // cluster reduction: ceil(m * 32 / S) quads (4 rows of one batch column) per CTA of the cluster
