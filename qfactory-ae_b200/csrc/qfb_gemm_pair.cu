@@ -22,7 +22,8 @@
 //
 // Measured (us, single-CTA kernel -> this): (28672,8192) at 256 / 1024 rows 137 -> 104 and 486 -> 375 (the latter 1.28
 // PFLOP/s and limited by power: 322 with the operands zeroed), (8192,8192) at 256 rows 64 -> 44, (12288,4096) at 1024
-// rows 125 -> 88, 8-bit (8192,8192) at 512 rows 81 -> 58.  Up to 128 columns it is slower than the single-CTA kernel
+// rows 125 -> 88, 8-bit (8192,8192) at 512 rows 81 -> 58 (launches in a row, workspaces with room to cut units; without it
+// every unit runs whole).  Up to 128 columns it is slower than the single-CTA kernel
 // (64 / 128 rows 81 / 85 against 63 / 77): the chain of hand-offs of a stage, longer across two CTAs, bounds both there.
 #include "qfb_common.cuh"
 #include "qfb_kernels.h"
