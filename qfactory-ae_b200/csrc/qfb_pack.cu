@@ -29,7 +29,7 @@ __device__ __forceinline__ int plane1_bit(int e) {
 // [row][k], four consecutive k to a word, whatever the source holds, and the packed words of either layout are put
 // together from there and leave in runs of 512 bytes.  HBM bound: the source is read once, coalesced along the
 // rows, and the packed bytes are written once.  Measured, (8192,28672) 4-bit from a checkpoint's words to the packed
-// layer: 62 us (3.9 TB/s of the 244 MB in and out); unpacking to int32, the range check and one thread per packed word
+// layer: 58 us (4.2 TB/s of the 244 MB in and out); unpacking to int32, the range check and one thread per packed word
 // took 1790.
 // Row stride 36 words: a multiple of 4, so that sixteen codes are one 16-byte store, and 4 (mod 32), so that the
 // fragment order's reads (8 rows x 4 words) and those stores meet no bank twice.

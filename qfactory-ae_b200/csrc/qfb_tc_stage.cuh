@@ -17,8 +17,8 @@ constexpr unsigned kSleepScale = 100, kSleepProducer = 100, kSleepMma = 20, kSle
 
 // Weight stages of 4- and 8-bit fragment layers arrive through a tensor map of 64-byte rows with the 64-byte swizzle.
 // As plain bytes the 32 lanes of a decode warp read words 64 bytes apart: 4-way bank conflicts on each of the 16
-// reads, 512 shared-memory cycles a stage beside the MMAs' and the copies' own ((28672,8192) at 64 / 1024 rows 67.5
-// -> 62 and 580 -> 491 us, (8192,28672) at 128 rows 85 -> 75 us).  Not for 2 bits, whose words are 32 bytes apart
+// reads, 512 shared-memory cycles a stage beside the MMAs' and the copies' own (launches in a row, (28672,8192) at 64 /
+// 1024 rows on one CTA 67.5 -> 62 and 580 -> 491 us, (8192,28672) at 128 rows 85 -> 75 us).  Not for 2 bits, whose words are 32 bytes apart
 // (2-way, and 32-byte rows would double the copy's requests), nor for 3, whose planes are read without conflicts
 // inside a row block; nor with per-stage accumulators (up to 32 rows), where it changes nothing ((8192,8192)
 // 8-bit at 24 rows 27.7 us with it, 27.6 without).
